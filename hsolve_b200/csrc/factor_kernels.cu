@@ -199,7 +199,7 @@ enum : int { kFail = 0, kOneJ = 1, kOneR = 2, kTwoR = 3, kNull = 4 };
 
 struct StepShared {
   int j, lim, prog, force, dec, r, stop;
-  int neg, pos, zero, two, forced, eb;
+  int neg, pos, zero, two, forced;
 };
 
 // Warp 0: decide the pivot at column j of the lower-stored matrix F (order m, ld ld) with
@@ -321,17 +321,14 @@ __device__ void elim2(R* F, int ld, int m, int j, R* tmp0, R* tmp1) {
   __syncthreads();
 }
 
-// Threshold Bunch-Kaufman on a lower-stored dense matrix in shared memory: candidates [0, nfs),
-// rows [0, m). root: pivots may be forced (never fail). Returns the number of eliminated columns
-// (positions [e, nfs) failed); pv[t] in {0 null, 1 1x1, 2/3 2x2}; lab follows the swaps.
+// One elimination of threshold Bunch-Kaufman on a lower-stored dense matrix in shared memory, from the
+// state in st: candidates [st.j, nfs), rows [0, m). root: pivots may be forced (never fail). Ends after
+// a pivot (st.j advanced) or with st.stop = 1 (nothing left, or positions [st.j, nfs) failed); pv[t] in
+// {0 null, 1 1x1, 2/3 2x2}; lab follows the swaps. The general step: runs of plain 1x1 pivots go
+// through fast_pivots.
 template <class R>
-__device__ int dense_bk(R* F, int ld, int m, int nfs, bool root, double u, double thr, int* lab, signed char* pv,
-                        R* tmp0, R* tmp1, StepShared& st) {
-  if (threadIdx.x == 0) {
-    st.j = 0; st.lim = nfs; st.prog = 0; st.force = 0; st.stop = 0;
-    st.neg = st.pos = st.zero = st.two = st.forced = 0;
-  }
-  __syncthreads();
+__device__ void dense_bk_step(R* F, int ld, int m, int nfs, bool root, double u, double thr, int* lab, signed char* pv,
+                              R* tmp0, R* tmp1, StepShared& st) {
   while (true) {
     if (threadIdx.x == 0) {
       st.stop = 0;
@@ -388,10 +385,9 @@ __device__ int dense_bk(R* F, int ld, int m, int nfs, bool root, double u, doubl
         if (st.lim < st.j) st.lim = st.j;
       }
     }
-    __syncthreads();
+    break;
   }
   __syncthreads();
-  return st.j;
 }
 
 // Warp maximum of non-negative floats: their bit patterns order like the values, so one integer
@@ -400,27 +396,116 @@ __device__ __forceinline__ float warp_maxf(float v) {
   return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
 }
 
-// One warp: threshold Bunch-Kaufman on the panel's diagonal block (order w <= 32, shared memory,
-// ld kNB, all rows candidates). Same acceptance rules as dense_bk; column maxima are reduced in
+// Runs of plain 1x1 pivots, the common case, by the whole CTA: the lower triangle (order m <= MAXM)
+// is in registers, column c in warp c % NW (slot c / NW), row i in lane i % 32. From st.j on, every
+// warp reads the pivot column from shared memory, takes the same decision from it and updates its own
+// columns; the owner of the next column publishes it (two buffers, so one block barrier per pivot).
+// Ends at st.lim or at the first column whose 1x1 test fails (nothing of that column is changed). The
+// column maximum is reduced in FP32, rounded up, so a pivot that passes here passes the test in FP64.
+//
+// A pivot is a chain of dependent operations (column read, 1 / d beside the maximum, update, write,
+// barrier), not work: one warp alone needed 1,400 cycles per pivot for the same block, most of them for the
+// update of its 32 columns one after another (the look-ahead step of a root panel of the n = 109,744 box:
+// 24.3 us with one warp, 12.7 us with the CTA; a whole count at n = 737, fronts up to 109: 735 -> 579 us).
+template <int MAXM, int NT, class R>
+__device__ __forceinline__ void fast_pivots(R (&y)[MAXM / (NT / 32)][MAXM / 32], R* buf, double u, double thr,
+                                            signed char* pv, StepShared& st) {
+  constexpr int NW = NT / 32, NC = MAXM / NW, NR = MAXM / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int j = st.j;
+  const int lim = st.lim;
+  auto publish = [&](int c) {
+    if ((c & (NW - 1)) != warp) return;
+    const int slot = c / NW;
+    R v[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) v[r] = y[0][r];
+#pragma unroll
+    for (int s = 1; s < NC; ++s)
+      if (slot == s) {
+#pragma unroll
+        for (int r = 0; r < NR; ++r) v[r] = y[s][r];
+      }
+#pragma unroll
+    for (int r = 0; r < NR; ++r) buf[(c & 1) * MAXM + lane + 32 * r] = v[r];
+  };
+  publish(j);
+  __syncthreads();
+  const int j0 = j;
+  int neg = 0;
+  const double nul = thr * (1.0 + 1e-6);
+  while (j < lim) {
+    const R* col = buf + (j & 1) * MAXM;
+    const R d = col[j];
+    R x[NR], yc[NC];
+    float g = 0.0f;
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      const int i = lane + 32 * r;
+      x[r] = i > j ? col[i] : R(0);
+      if constexpr (sizeof(R) == 8) g = fmaxf(g, __double2float_ru(fabs(x[r])));
+      else g = fmaxf(g, fabsf(x[r]));
+    }
+#pragma unroll
+    for (int s = 0; s < NC; ++s) yc[s] = col[warp + NW * s];
+    const R inv = R(1) / d;
+    const double gc = warp_maxf(g);
+    const double dcc = fabs(static_cast<double>(d));
+    if (!(dcc > 0.0 && dcc >= u * gc) || (thr >= 0.0 && fmax(dcc, gc) <= nul)) break;
+#pragma unroll
+    for (int r = 0; r < NR; ++r) x[r] *= inv;
+#pragma unroll
+    for (int s = 0; s < NC; ++s)
+      if (warp + NW * s > j) {
+#pragma unroll
+        for (int r = 0; r < NR; ++r) y[s][r] -= x[r] * yc[s];
+      }
+    if (j + 1 < lim) publish(j + 1);
+    if ((j & (NW - 1)) == warp) {
+#pragma unroll
+      for (int s = 0; s < NC; ++s)
+        if (j / NW == s) {
+#pragma unroll
+          for (int r = 0; r < NR; ++r)
+            if (lane + 32 * r > j) y[s][r] = x[r];
+        }
+    }
+    if (threadIdx.x == 0) pv[j] = 1;
+    if (d < R(0)) ++neg;
+    ++j;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0 && j > j0) {
+    st.neg += neg;
+    st.pos += j - j0 - neg;
+    st.j = j;
+    st.prog = 1;
+  }
+  __syncthreads();
+}
+
+// One warp: one elimination of threshold Bunch-Kaufman on the panel's diagonal block (order w <= 32,
+// shared memory, ld kNB, all rows candidates), from the state in st: the general step, for the columns
+// where fast_pivots stops. Same acceptance rules as dense_bk_step; column maxima are reduced in
 // single precision (a threshold test needs no more), the argmax for a 2 x 2 partner only when the
 // 1 x 1 test fails, one reciprocal per pivot. The update of a step reads the pivot column(s) into
-// registers first, so its column read-modify-writes are independent and pipeline (and the routine
-// stays a compact loop: it runs once per panel, from a cold instruction cache). Not inlined: as a
-// function of its own it is register-allocated apart from the panel kernels' other phases (255
-// registers), which measured faster than the inlined loop; the call is once per panel.
-// Warp-synchronous: no block barriers. Returns the eliminated count; [e, w) could not be pivoted.
+// registers first, so its column read-modify-writes are independent and pipeline. Not inlined: as a
+// function of its own it is register-allocated apart from the panel kernels' other phases.
+// Warp-synchronous: no block barriers. Ends after a pivot or with st.stop = 1 ([st.j, w) could not be
+// pivoted).
 template <class R>
-__device__ __noinline__ int warp_block_bk(R* F, int w, bool root, double u, double thr, int* lab, signed char* pv,
-                                          StepShared& st, int j0 = 0, int prog0 = 0) {
+__device__ __noinline__ void warp_block_step(R* F, int w, bool root, double u, double thr, int* lab, signed char* pv,
+                                             StepShared& st) {
   const int lane = threadIdx.x & 31;
   constexpr int ld = kNB;
   __shared__ R s_c0[kNB], s_c1[kNB];
-  int j = j0, lim = w, prog = prog0, force = 0;
+  int j = st.j, lim = st.lim, prog = st.prog, force = st.force, stop = 0;
   int neg = 0, pos = 0, zero = 0, two = 0, forced = 0;
   while (j < w) {
     if (j >= lim) {
       if (prog) { lim = w; prog = 0; continue; }
       if (root && !force) { force = 1; lim = w; continue; }
+      stop = 1;
       break;
     }
     const R* cj = F + j * ld;
@@ -537,43 +622,99 @@ __device__ __noinline__ int warp_block_bk(R* F, int w, bool root, double u, doub
     prog = 1;
     force = 0;
     if (lim < j) lim = j;
+    break;
   }
-  if (lane == 0) { st.neg += neg; st.pos += pos; st.zero += zero; st.two += two; st.forced += forced; }
-  return j;
+  if (lane == 0) {
+    st.neg += neg; st.pos += pos; st.zero += zero; st.two += two; st.forced += forced;
+    st.j = j; st.lim = lim; st.prog = prog; st.force = force; st.stop = stop;
+  }
+}
+
+__device__ __forceinline__ void bk_begin(StepShared& st, int lim) {
+  st.j = 0; st.lim = lim; st.prog = 0; st.force = 0; st.stop = 0;
+  st.neg = st.pos = st.zero = st.two = st.forced = 0;
+}
+
+// The panel's diagonal block by the whole CTA: y holds its lower triangle (row lane, columns
+// warp + 8 s); st was begun (and a block barrier passed) before. The factored block is left in F
+// (shared, ld kNB, lower triangle).
+template <class R>
+__device__ void block_bk(R (&y)[4][1], R* F, R* buf, int w, bool root, double u, double thr, int* lab, signed char* pv,
+                         StepShared& st) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  while (true) {
+    if (!st.force && st.j < st.lim) fast_pivots<kNB, kAppThreads>(y, buf, u, thr, pv, st);
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int c = warp + 8 * s;
+      if (lane >= c && lane < w) F[lane + c * kNB] = y[s][0];
+    }
+    __syncthreads();
+    if (st.j >= w) break;
+    if (warp == 0) warp_block_step(F, w, root, u, thr, lab, pv, st);
+    __syncthreads();
+    if (st.stop || st.j >= w) break;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int c = warp + 8 * s;
+      if (lane >= c && lane < w) y[s][0] = F[lane + c * kNB];
+    }
+  }
 }
 
 }  // namespace
 
 // ---------------------------------------------------------------------- small fronts (smem)
 
-template <int MAXM, class R>
-__global__ void __launch_bounds__(256) k_front_small(const std::int32_t* list, const SnDev* sn, R* panels,
-                                                      R* cb, signed char* piv_out, std::int32_t* pidx_out,
-                                                      FactorParams prm, FactorCounters* cnt, std::int32_t* failed) {
+// A front in registers: column c in warp c % NW, row i in lane i % 32 (fast_pivots); shared memory holds
+// it only for the general pivot steps (2x2 pivots, swaps, null and forced pivots).
+template <int MAXM, int NT, class R>
+__global__ void __launch_bounds__(NT) k_front_small(const std::int32_t* list, const SnDev* sn, R* panels, R* cb,
+                                                    signed char* piv_out, std::int32_t* pidx_out, FactorParams prm,
+                                                    FactorCounters* cnt, std::int32_t* failed) {
+  constexpr int NW = NT / 32, NC = MAXM / NW, NR = MAXM / 32;
   extern __shared__ __align__(16) unsigned char small_dyn[];
   R* F = reinterpret_cast<R*>(small_dyn);
-  __shared__ R tmp0[MAXM], tmp1[MAXM];
+  __shared__ R tmp0[MAXM], tmp1[MAXM], buf[2 * MAXM];
   __shared__ int lab[MAXM];
   __shared__ signed char pv[MAXM];
   __shared__ StepShared st;
   const SnDev d = sn[list[blockIdx.x]];
-  const int m = d.m, k = d.k, ld = m, c = m - k;
-  for (int t = threadIdx.x; t < m * m; t += blockDim.x) {
-    const int i = t % m, j = t / m;
-    if (i < j) continue;
-    F[t] = j < k ? panels[d.panel_off + static_cast<std::int64_t>(j) * m + i]
-                 : cb[d.cb_off + static_cast<std::int64_t>(j - k) * c + (i - k)];
-  }
-  for (int t = threadIdx.x; t < m; t += blockDim.x) lab[t] = t;
+  const int m = d.m, k = d.k, ld = m;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  R* panel = panels + d.panel_off;
+  R* cbb = cb + d.cb_off;
+  // the lower triangle's entries of this thread: f(entry, pointer in the front's storage, i, c)
+  R y[NC][NR];
+  auto each = [&](auto&& f) {
+#pragma unroll
+    for (int s = 0; s < NC; ++s) {
+      const int c = warp + NW * s;
+      R* col = c < k ? panel + static_cast<std::int64_t>(c) * m : cbb + static_cast<std::int64_t>(c - k) * (m - k) - k;
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        const int i = lane + 32 * r;
+        f(y[s][r], col, i, c, c < m && i >= c && i < m);
+      }
+    }
+  };
+  each([&](R& v, const R* col, int i, int, bool in) { v = in ? col[i] : R(0); });
+  for (int t = threadIdx.x; t < m; t += NT) lab[t] = t;
+  if (threadIdx.x == 0) bk_begin(st, k);
   __syncthreads();
   const double thr = null_threshold(prm);
-  const int e = dense_bk(F, ld, m, k, d.parent < 0, prm.u, thr, lab, pv, tmp0, tmp1, st);
-  for (int t = threadIdx.x; t < m * m; t += blockDim.x) {
-    const int i = t % m, j = t / m;
-    if (i < j) continue;
-    if (j < k) panels[d.panel_off + static_cast<std::int64_t>(j) * m + i] = F[t];
-    else cb[d.cb_off + static_cast<std::int64_t>(j - k) * c + (i - k)] = F[t];
+  while (true) {
+    if (!st.force && st.j < st.lim) fast_pivots<MAXM, NT>(y, buf, prm.u, thr, pv, st);
+    if (st.j >= k) break;
+    each([&](R& v, const R*, int i, int c, bool in) { if (in) F[i + c * ld] = v; });
+    __syncthreads();
+    dense_bk_step(F, ld, m, k, d.parent < 0, prm.u, thr, lab, pv, tmp0, tmp1, st);
+    each([&](R& v, const R*, int i, int c, bool in) { if (in) v = F[i + c * ld]; });
+    if (st.stop) break;
+    __syncthreads();  // every column is read before a later step writes the matrix again
   }
+  const int e = st.j;
+  each([&](const R& v, R* col, int i, int, bool in) { if (in) col[i] = v; });
   for (int t = threadIdx.x; t < k; t += blockDim.x) {
     pidx_out[d.first + t] = lab[t];
     piv_out[d.first + t] = t < e ? pv[t] : static_cast<signed char>(-1);
@@ -725,8 +866,8 @@ __device__ void app_init(AppFront<R>& F, int rank, int nr) {
 // Rank 0: decide what the next panel is (stop = 1: front finished), and factorize its diagonal block
 // with block-restricted threshold Bunch-Kaufman; permute the L rows of the block; publish to scratch.
 template <class R>
-__device__ void app_control_and_block(AppFront<R>& F, const FactorParams& prm, double thr, R* Bs, R* tmp0,
-                                      R* tmp1, int* slab, signed char* spv, StepShared& bst, int* shared_stop,
+__device__ void app_control_and_block(AppFront<R>& F, const FactorParams& prm, double thr, R* Bs, R* tmp,
+                                      int* slab, signed char* spv, StepShared& bst, int* shared_stop,
                                       FactorCounters* cnt, std::int32_t* failed, int* level_done) {
   AppCtrl* c = F.ctrl;
   const int k = F.f.k;
@@ -804,23 +945,24 @@ __device__ void app_control_and_block(AppFront<R>& F, const FactorParams& prm, d
     if (r > p + 1) front_swap(F.f, p + 1, r, F.plab);
     __syncthreads();
   }
-  for (int t = threadIdx.x; t < w * w; t += blockDim.x) {
-    const int i = t % w, j = t / w;
-    if (i >= j) {
-      const double v = F.f.at(p + i, p + j);
-      Bs[i + j * kNB] = v;
-      F.Borig[i + j * kNB] = v;
-    }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  R y[4][1];
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    const int c2 = warp + 8 * s;
+    const bool in = lane >= c2 && lane < w;
+    y[s][0] = in ? F.f.at(p + lane, p + c2) : R(0);
+  }
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    const int c2 = warp + 8 * s;
+    if (lane >= c2 && lane < w) F.Borig[lane + c2 * kNB] = y[s][0];
   }
   for (int t = threadIdx.x; t < w; t += blockDim.x) slab[t] = t;
-  if (threadIdx.x == 0) { bst.neg = bst.pos = bst.zero = bst.two = bst.forced = 0; bst.eb = 0; }
+  if (threadIdx.x == 0) bk_begin(bst, w);
   __syncthreads();
-  if (threadIdx.x < 32) {
-    const int e = warp_block_bk(Bs, w, force, prm.u, thr, slab, spv, bst);
-    if (threadIdx.x == 0) bst.eb = e;
-  }
-  __syncthreads();
-  const int eb = bst.eb;
+  block_bk(y, Bs, tmp, w, force, prm.u, thr, slab, spv, bst);
+  const int eb = bst.j;
   if (__syncthreads_or(threadIdx.x < w && slab[threadIdx.x] != static_cast<int>(threadIdx.x))) {
     // the block's rows were swapped: its pivot labels follow
     int old = 0;
@@ -828,11 +970,12 @@ __device__ void app_control_and_block(AppFront<R>& F, const FactorParams& prm, d
     __syncthreads();
     if (threadIdx.x < w) F.plab[p + threadIdx.x] = old;
   }
-  for (int t = threadIdx.x; t < w * w; t += blockDim.x) {
-    const int i = t % w, j = t / w;
-    if (i >= j) F.f.at(p + i, p + j) = Bs[i + j * kNB];
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    const int c2 = warp + 8 * s;
+    if (lane >= c2 && lane < w) F.f.at(p + lane, p + c2) = Bs[lane + c2 * kNB];
+    F.B[lane + c2 * kNB] = Bs[lane + c2 * kNB];
   }
-  for (int t = threadIdx.x; t < kNB * kNB; t += blockDim.x) F.B[t] = Bs[t];
   for (int t = threadIdx.x; t < kNB; t += blockDim.x) {
     F.lab[t] = slab[t];
     F.pv[t] = spv[t];
@@ -1337,7 +1480,7 @@ __device__ void app_advance(AppFront<R>& F, int q) {
 template <class R>
 struct AppSmem {
   R Bs[kNB * kNB];
-  R tmp0[kNB], tmp1[kNB];
+  R tmp[2 * kNB];
   int slab[kNB];
   signed char spv[kNB];
   unsigned long long scm[kNB], srm[kNB];
@@ -1414,7 +1557,7 @@ __device__ void app_front(AppFront<R>& F, int rank, int nr, const FactorParams& 
       if (rank == 0) {
         if (j > 0) app_advance(F, qprev);
         set_slot(F, j & 1);
-        app_control_and_block(F, prm, thr, sm.Bs, sm.tmp0, sm.tmp1, sm.slab, sm.spv, sm.bst, &sm.stop, cnt, failed,
+        app_control_and_block(F, prm, thr, sm.Bs, sm.tmp, sm.slab, sm.spv, sm.bst, &sm.stop, cnt, failed,
                               level_done);
       }
       if (!sync()) break;
@@ -1435,7 +1578,7 @@ __device__ void app_front(AppFront<R>& F, int rank, int nr, const FactorParams& 
       __syncthreads();
       app_advance(F, q);
       set_slot(F, (j + 1) & 1);
-      app_control_and_block(F, prm, thr, sm.Bs, sm.tmp0, sm.tmp1, sm.slab, sm.spv, sm.bst, &sm.stop, cnt, failed,
+      app_control_and_block(F, prm, thr, sm.Bs, sm.tmp, sm.slab, sm.spv, sm.bst, &sm.stop, cnt, failed,
                             level_done);
     }
     if (!sync()) break;
@@ -1568,8 +1711,8 @@ void launch_front_small(int maxm, const std::int32_t* list, int nlist, const SnD
   if (nlist <= 0) return;
   const std::size_t smem = static_cast<std::size_t>(maxm) * maxm * sizeof(R);
   note_launches(1);
-  if (maxm <= 32) k_front_small<32, R><<<nlist, 128, smem, s>>>(list, sn, panels, cb, piv, pidx, prm, cnt, failed);
-  else k_front_small<kSmallMax, R><<<nlist, 256, smem, s>>>(list, sn, panels, cb, piv, pidx, prm, cnt, failed);
+  if (maxm <= 32) k_front_small<32, 128, R><<<nlist, 128, smem, s>>>(list, sn, panels, cb, piv, pidx, prm, cnt, failed);
+  else k_front_small<kSmallMax, 256, R><<<nlist, 256, smem, s>>>(list, sn, panels, cb, piv, pidx, prm, cnt, failed);
 }
 
 template <class R>
