@@ -782,6 +782,7 @@ struct AppFront {
   unsigned long long* cmax;
   unsigned long long* rmax;
   R* backup;       // kNB columns of m rows
+  R* wd;           // W = L D of the pending pivots: column s is pivot fb + s, m rows each
   std::int32_t* plab;
   signed char* ppv;
 };
@@ -828,6 +829,8 @@ __device__ AppFront<R> make_front(const SnDev& d, R* panels, R* cb, double* scra
   F.slots = s;
   s += 2 * kAppSlotDoubles;
   F.backup = reinterpret_cast<R*>(s);
+  s += static_cast<std::int64_t>(d.m) * kNB;
+  F.wd = reinterpret_cast<R*>(s);
   F.plab = pidx_out + d.first;
   F.ppv = piv_out + d.first;
   set_slot(F, 0);
@@ -1103,6 +1106,11 @@ __device__ void app_rows(AppFront<R>& F, const StepView& v, int rank, int nr, R*
         for (int s2 = 0; s2 < t; ++s2) acc = fma(-y[s2], Lm[t * kNB + s2], acc);
         y[t] = acc;
       }
+      // the substituted row is W = L D, the update's second operand (zero for a null pivot)
+      R* wrow = F.wd + static_cast<std::int64_t>(p - v.fb) * m + c0 + r;
+#pragma unroll
+      for (int t = 0; t < kNB; ++t)
+        if (t < eb) wrow[static_cast<std::int64_t>(t) * m] = ksel[t] == 1 ? R(0) : y[t];
       R prev = R(0);
 #pragma unroll
       for (int t = 0; t < kNB; ++t) {
@@ -1233,7 +1241,8 @@ __device__ int app_accept(AppFront<R>& F, const StepView& v, int rank, double th
 
 // All ranks: restore the rejected block columns [q, w) from the backup / original block.
 template <class R>
-__device__ void app_restore(AppFront<R>& F, const StepView& v, int rank, int nr, int q) {
+__device__ void app_restore(AppFront<R>& F, const StepView& v, int rank, int nr, int q, const R* Bs,
+                            const signed char* spv) {
   const int p = v.p, w = v.w, m = F.f.m;
   const int rtotal = m - (p + w);
   const int rchunk = (rtotal + nr - 1) / nr;
@@ -1246,6 +1255,16 @@ __device__ void app_restore(AppFront<R>& F, const StepView& v, int rank, int nr,
       if (b >= q && a >= b) {
         const int la = F.lab[a], lb = F.lab[b];
         F.f.at(p + a, p + b) = la >= lb ? F.Borig[la + lb * kNB] : F.Borig[lb + la * kNB];
+      }
+      if (a >= q && b < q) {
+        // W = L D of the rejected rows, which the row step did not see (a 2x2 pivot's coupling is D)
+        const R l = Bs[a + b * kNB];
+        const signed char ty = spv[b];
+        R x = R(0);
+        if (ty == 1) x = l * Bs[b + b * kNB];
+        else if (ty == 2) x = fma(Bs[b + b * kNB], l, Bs[b + 1 + b * kNB] * Bs[a + (b + 1) * kNB]);
+        else if (ty == 3) x = fma(Bs[b + (b - 1) * kNB], Bs[a + (b - 1) * kNB], Bs[b + b * kNB] * l);
+        F.wd[static_cast<std::int64_t>(p - v.fb + b) * m + p + a] = x;
       }
     }
   }
@@ -1269,32 +1288,33 @@ __device__ __forceinline__ bool app_flushes(int p, int w, int q, int lim, int fb
 // All ranks: C(i, c) -= sum_{s in [fb, p+q)} L(i, s) W(c, s), W = L D, over the lower triangle
 // c <= i < m of the columns c in [p+q, col_hi): all trailing columns when the step flushes, else the
 // next panel's. Rejected columns [p+q, p+w) of a flushing panel already hold the updates of
-// [fb, p) (they were part of the panel) and take only those of [p, p+q). W is formed while staging
-// from L and the pivots' D (1x1: d; 2x2 [a b; b c]: W(c, s) = a L(c, s) + b L(c, s+1) and
-// W(c, s+1) = b L(c, s) + c L(c, s+1)); null pivots have L = 0.
+// [fb, p) (they were part of the panel) and take only those of [p, p+q). W is what the row step's
+// substitution leaves before D^-1 (kept in the front's scratch); null pivots have L = 0.
 //
 // The update runs on the FP64 tensor cores (mma.sync m8n8k4, D = A B + C with A 8 x 4, B 4 x 8) by
-// 64 x 64 tiles of C dealt round-robin to the ranks: the tile's rows of L and its columns' rows of
-// L (<= kKB pivots) are copied asynchronously (cp.async, zero-filled outside the front) into shared
-// memory, column-major with stride kUpdLd = 4 (mod 16), so that the copies of consecutive rows are
-// contiguous and every fragment read of a half-warp hits 32 distinct banks; D is then applied to the
-// second copy in place. Warp w (of 8) computes rows 16 (w % 4) .. +16 and columns 32 (w / 4) .. +32
+// 64 x 64 tiles of C dealt round-robin to the ranks. The tile's rows of L and its columns' rows of
+// W come in chunks of kUpdChunk pivots by cp.async (zero-filled outside the front), column-major with
+// stride kUpdLd = 4 (mod 16): copies of consecutive rows are contiguous and every fragment read of a
+// half-warp hits 32 distinct banks. kUpdStages chunks are in flight across tile boundaries, so the
+// next tile arrives while this one is computed (a 64 x 64 x 128 tile is 4.5 us of FP64 tensor work on
+// an SM; staged as a whole, scaled by D and only then multiplied, the update phase of a root panel of
+// the n = 109,744 box took 20.0 us, now 16.1; factorize + 8 solves there 21.4 -> 18.5 ms).
+// Warp w (of 8) computes rows 16 (w % 4) .. +16 and columns 32 (w / 4) .. +32
 // of the tile as 2 x 4 blocks of 8 x 8. A thread's fragment element (g, t) is row g = lane / 4,
 // column t = lane % 4 of A; row t, column g of B; row g, columns 2t, 2t + 1 of C.
 // FP32 factors (the operator factorization of the mixed-precision path) keep the same staging and
 // the same output ownership per thread, and accumulate with FP32 FMAs (there is no FP32 tensor
 // instruction with full FP32 operands; the FP64 refinement of every solve absorbs FP32 rounding).
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-}
-
 //
 // With look-ahead (la: the panel was accepted whole and the next one follows directly), rank 0 takes
 // only tile 0, which holds the next panel's diagonal block, so that it can factorize that block
 // while the other ranks finish the remaining tiles.
+struct UpdTile {
+  int tile, i0, j0;
+};
+
 template <class R>
-__device__ void app_update(AppFront<R>& F, const StepView& v, int rank, int nr, int q, bool la, R* Ls, R* Ws,
-                           R* ca, R* cb, int* cd, const R* Bs, const signed char* spv) {
+__device__ void app_update(AppFront<R>& F, const StepView& v, int rank, int nr, int q, bool la, R* stage) {
   const int p = v.p, w = v.w, lim = v.lim, fb = v.fb, m = F.f.m;
   const int from = p + q;
   const int K = from - fb;
@@ -1303,29 +1323,6 @@ __device__ void app_update(AppFront<R>& F, const StepView& v, int rank, int nr, 
   const bool flush = app_flushes(p, w, q, lim, fb);
   const int col_hi = flush ? m : min(m, from + min(kNB, lim - from));
   const int rej_hi = flush && q < w ? p + w : 0;  // columns below this take only the pivots >= p
-  // staging coefficients of the pending pivots: W(c, fb+s) = ca[s] L(c, fb+s) + cb[s] L(c, fb+s+cd[s])
-  // (the panel's own pivots from the block in shared memory: rank 0 books their types in global
-  // memory while the other ranks may already be here)
-  for (int s = threadIdx.x; s < K; s += blockDim.x) {
-    const int j = fb + s;
-    R x = R(0), y = R(0);
-    int d = 0;
-    if (j >= p) {
-      const int t = j - p;
-      const signed char ty = spv[t];
-      if (ty == 1) x = Bs[t + t * kNB];
-      else if (ty == 2) { x = Bs[t + t * kNB]; y = Bs[t + 1 + t * kNB]; d = 1; }
-      else if (ty == 3) { x = Bs[t + t * kNB]; y = Bs[t + (t - 1) * kNB]; d = -1; }
-    } else {
-      const signed char ty = __ldcg(&F.ppv[j]);
-      if (ty == 1) x = __ldcg(&F.f.at(j, j));
-      else if (ty == 2) { x = __ldcg(&F.f.at(j, j)); y = __ldcg(&F.f.at(j + 1, j)); d = 1; }
-      else if (ty == 3) { x = __ldcg(&F.f.at(j, j)); y = __ldcg(&F.f.at(j, j - 1)); d = -1; }
-    }
-    ca[s] = x;
-    cb[s] = y;
-    cd[s] = d;
-  }
   const int nt = (rows + kTile - 1) / kTile;
   const int nct = (col_hi - from + kTile - 1) / kTile;
   const int ntiles = nct * nt - nct * (nct - 1) / 2;
@@ -1333,109 +1330,125 @@ __device__ void app_update(AppFront<R>& F, const StepView& v, int rank, int nr, 
   const int g = lane >> 2, t4 = lane & 3;
   const int rbase = (warp & 3) * 16, cbase = (warp >> 2) * 32;
   const int Kpad = (K + 3) & ~3;
+  const int nk = (K + kUpdChunk - 1) / kUpdChunk;
   // tiles of this rank: round-robin, or with look-ahead tile 0 for rank 0 and the rest over ranks 1..
   const bool split = la && nr > 1;
   const int tfirst = split ? (rank == 0 ? 0 : rank) : rank;
   const int tstep = split ? (rank == 0 ? ntiles : nr - 1) : nr;
-  for (int tile = tfirst; tile < ntiles; tile += tstep) {
+  if (tfirst >= ntiles) return;
+  auto locate = [&](UpdTile& t) {
     int ti, tj;
     if (nct == nt) {
-      ti = static_cast<int>((sqrt(8.0 * tile + 1.0) - 1.0) * 0.5);
-      while ((ti + 1) * (ti + 2) / 2 <= tile) ++ti;
-      while (ti * (ti + 1) / 2 > tile) --ti;
-      tj = tile - ti * (ti + 1) / 2;
+      ti = static_cast<int>((sqrtf(8.0f * static_cast<float>(t.tile) + 1.0f) - 1.0f) * 0.5f);
+      while ((ti + 1) * (ti + 2) / 2 <= t.tile) ++ti;
+      while (ti * (ti + 1) / 2 > t.tile) --ti;
+      tj = t.tile - ti * (ti + 1) / 2;
     } else {
-      int rest = tile;
+      int rest = t.tile;
       tj = 0;
       while (rest >= nt - tj) { rest -= nt - tj; ++tj; }
       ti = tj + rest;
     }
-    const int i0 = from + ti * kTile, j0 = from + tj * kTile;
-    __syncthreads();
-    {
-      // thread: tile row r, pivots s = sg, sg + 4, ...: all copies in flight at once
-      const int r = threadIdx.x & (kTile - 1), sg = threadIdx.x >> 6;
-      const int i = i0 + r, cc = j0 + r;
-      const int li = i < m ? i : from, lc = cc < m ? cc : from;
-      const bool lb = i < m, wb = cc < col_hi;
-#pragma unroll 8
-      for (int s = sg; s < Kpad; s += kAppThreads / kTile) {
-        const bool in = s < K;
-        const R* lj = F.f.col(fb + (in ? s : 0));
-        cp_async_elem(&Ls[s * kUpdLd + r], lj + li, in && lb);
-        cp_async_elem(&Ws[s * kUpdLd + r], lj + lc, in && wb);
+    t.i0 = from + ti * kTile;
+    t.j0 = from + tj * kTile;
+  };
+  // chunk `kc` of tile `t` into stage `st`: a thread copies tile row r, pivots sg, sg + 4, ...
+  const R* lpan = F.f.panel + static_cast<std::int64_t>(fb) * m;
+  const int r = threadIdx.x & (kTile - 1), sg = threadIdx.x >> 6;
+  auto issue = [&](const UpdTile& t, int kc, int st) {
+    R* Ls = stage + st * (2 * kUpdChunk * kUpdLd);
+    R* Ws = Ls + kUpdChunk * kUpdLd;
+    const int i = t.i0 + r, c = t.j0 + r;
+    const int li = i < m ? i : from, lc = c < col_hi ? c : from;
+    const int smin = c < rej_hi ? p - fb : 0;
+#pragma unroll
+    for (int u = 0; u < kUpdChunk / 4; ++u) {
+      const int sl = sg + 4 * u, s = kc * kUpdChunk + sl;
+      if (s >= Kpad) break;
+      const bool in = s < K;
+      const std::int64_t col = static_cast<std::int64_t>(in ? s : 0) * m;
+      cp_async_elem(&Ls[sl * kUpdLd + r], lpan + col + li, in && i < m);
+      cp_async_elem(&Ws[sl * kUpdLd + r], F.wd + col + lc, in && c < col_hi && s >= smin);
+    }
+  };
+  UpdTile ft{tfirst, 0, 0}, ct;  // the tile being fetched, and the one computed
+  locate(ft);
+  ct = ft;
+  int fk = 0, fst = 0, cst = 0;
+  auto fetch_next = [&]() {
+    if (ft.tile < ntiles) {
+      issue(ft, fk, fst);
+      fst = fst + 1 == kUpdStages ? 0 : fst + 1;
+      if (++fk == nk) {
+        fk = 0;
+        ft.tile += tstep;
+        if (ft.tile < ntiles) locate(ft);
       }
     }
-    // prefetch this thread's C entries (rows rbase + 8a + g, columns cbase + 8b + 2 t4 + e)
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  __syncthreads();  // the staging area's last users are done
+#pragma unroll
+  for (int u = 0; u < kUpdStages - 1; ++u) fetch_next();
+  while (ct.tile < ntiles) {
+    const int i0 = ct.i0, j0 = ct.j0;
+    // warps whose 32 columns all lie at or beyond col_hi (the second half of a panel's tile) or
+    // whose 16 rows all lie above their first column have nothing to update
+    const bool idle = j0 + cbase >= col_hi || i0 + rbase + 15 < j0 + cbase;
+    // this thread's C entries (rows rbase + 8a + g, columns cbase + 8b + 2 t4 + e)
     R* colp[4][2];
-    R cv[2][4][2];
+    R cv[2][4][2], acc[2][4][2];
 #pragma unroll
     for (int b = 0; b < 4; ++b)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int cc = j0 + cbase + 8 * b + 2 * t4 + e;
-        colp[b][e] = cc < col_hi ? F.f.col(cc) : nullptr;
+        colp[b][e] = !idle && cc < col_hi ? F.f.col(cc) : nullptr;
 #pragma unroll
         for (int a = 0; a < 2; ++a) {
           const int i = i0 + rbase + 8 * a + g;
           cv[a][b][e] = (colp[b][e] && i < m && cc <= i) ? colp[b][e][i] : R(0);
+          acc[a][b][e] = R(0);
         }
       }
-    cp_async_wait_all();
-    __syncthreads();
-    // W = L D in place (a 2x2 pair by its first column), zero for the rejected columns' old pivots
-    for (int t = threadIdx.x; t < K * kTile; t += blockDim.x) {
-      const int s = t / kTile, r = t % kTile;
-      const int d = cd[s];
-      if (d < 0) continue;
-      const bool masked = j0 + r < rej_hi && fb + s < p;
-      R* w0 = &Ws[s * kUpdLd + r];
-      if (d == 0) {
-        *w0 = masked ? R(0) : ca[s] * *w0;
-      } else {
-        R* w1 = w0 + kUpdLd;
-        const R x0 = *w0, x1 = *w1;
-        *w0 = masked ? R(0) : fma(ca[s], x0, cb[s] * x1);
-        *w1 = masked ? R(0) : fma(cb[s + 1], x0, ca[s + 1] * x1);
-      }
-    }
-    __syncthreads();
-    // warps whose 32 columns all lie at or beyond col_hi (the second half of a panel's tile) or
-    // whose 16 rows all lie above their first column have nothing to update
-    const bool idle = j0 + cbase >= col_hi || i0 + rbase + 15 < j0 + cbase;
-    if (idle) continue;
-    R acc[2][4][2];
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) { acc[a][b][0] = R(0); acc[a][b][1] = R(0); }
-    if constexpr (sizeof(R) == 8) {
+    for (int kc = 0; kc < nk; ++kc) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kUpdStages - 2) : "memory");
+      __syncthreads();  // the chunk has arrived for every thread, and the stage fetched next is free
+      fetch_next();
+      const R* Ls = stage + cst * (2 * kUpdChunk * kUpdLd);
+      const R* Ws = Ls + kUpdChunk * kUpdLd;
+      cst = cst + 1 == kUpdStages ? 0 : cst + 1;
+      if (idle) continue;
+      if constexpr (sizeof(R) == 8) {
+        const int send = min(kUpdChunk, Kpad - kc * kUpdChunk);
 #pragma unroll 2
-      for (int s0 = 0; s0 < Kpad; s0 += 4) {
-        double af[2], bf[4];
+        for (int s0 = 0; s0 < send; s0 += 4) {
+          double af[2], bf[4];
 #pragma unroll
-        for (int a = 0; a < 2; ++a) af[a] = Ls[(s0 + t4) * kUpdLd + rbase + 8 * a + g];
+          for (int a = 0; a < 2; ++a) af[a] = Ls[(s0 + t4) * kUpdLd + rbase + 8 * a + g];
 #pragma unroll
-        for (int b = 0; b < 4; ++b) bf[b] = Ws[(s0 + t4) * kUpdLd + cbase + 8 * b + g];
+          for (int b = 0; b < 4; ++b) bf[b] = Ws[(s0 + t4) * kUpdLd + cbase + 8 * b + g];
 #pragma unroll
-        for (int a = 0; a < 2; ++a)
+          for (int a = 0; a < 2; ++a)
 #pragma unroll
-          for (int b = 0; b < 4; ++b) dmma_m8n8k4(acc[a][b][0], acc[a][b][1], af[a], bf[b]);
-      }
-    } else {
-      // FP32: the thread's own 2 x 8 outputs by rank-1 steps (two L values, four W pairs per pivot)
+            for (int b = 0; b < 4; ++b) dmma_m8n8k4(acc[a][b][0], acc[a][b][1], af[a], bf[b]);
+        }
+      } else {
+        // FP32: the thread's own 2 x 8 outputs by rank-1 steps (two L values, four W pairs per pivot)
+        const int send = min(kUpdChunk, K - kc * kUpdChunk);
 #pragma unroll 4
-      for (int s = 0; s < K; ++s) {
-        const R* ls = Ls + s * kUpdLd + rbase + g;
-        const R* ws = Ws + s * kUpdLd + cbase + 2 * t4;
-        const R l0 = ls[0], l1 = ls[8];
+        for (int s = 0; s < send; ++s) {
+          const R* ls = Ls + s * kUpdLd + rbase + g;
+          const R* ws = Ws + s * kUpdLd + cbase + 2 * t4;
+          const R l0 = ls[0], l1 = ls[8];
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const auto w2 = load_pair(ws + 8 * b);
-          acc[0][b][0] = fma(l0, w2.x, acc[0][b][0]);
-          acc[0][b][1] = fma(l0, w2.y, acc[0][b][1]);
-          acc[1][b][0] = fma(l1, w2.x, acc[1][b][0]);
-          acc[1][b][1] = fma(l1, w2.y, acc[1][b][1]);
+          for (int b = 0; b < 4; ++b) {
+            const auto w2 = load_pair(ws + 8 * b);
+            acc[0][b][0] = fma(l0, w2.x, acc[0][b][0]);
+            acc[0][b][1] = fma(l0, w2.y, acc[0][b][1]);
+            acc[1][b][0] = fma(l1, w2.x, acc[1][b][0]);
+            acc[1][b][1] = fma(l1, w2.y, acc[1][b][1]);
+          }
         }
       }
     }
@@ -1450,7 +1463,10 @@ __device__ void app_update(AppFront<R>& F, const StepView& v, int rank, int nr, 
           if (colp[b][e] && i < m && cc <= i) colp[b][e][i] = cv[a][b][e] - acc[a][b][e];
         }
       }
+    ct.tile += tstep;
+    if (ct.tile < ntiles) locate(ct);
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 // Rank 0: advance past the accepted pivots; move rejected columns behind the candidates.
@@ -1485,8 +1501,6 @@ struct AppSmem {
   signed char spv[kNB];
   unsigned long long scm[kNB], srm[kNB];
   StepShared bst;
-  R ca[kKB], cb[kKB];
-  int cd[kKB];
   int stop, q, ok;
 };
 
@@ -1541,7 +1555,7 @@ __device__ bool front_barrier(int* bar, int nr, unsigned long long* timeouts, in
 // block's arrays never overlap the ones slower CTAs still read.
 template <bool kCoop, class R>
 __device__ void app_front(AppFront<R>& F, int rank, int nr, const FactorParams& prm, FactorCounters* cnt,
-                          std::int32_t* failed, int* level_done, AppSmem<R>& sm, R* Ls, R* Ws) {
+                          std::int32_t* failed, int* level_done, AppSmem<R>& sm, R* stage) {
   const double thr = null_threshold(prm);
   const double inv_u = 1.0 / prm.u;
   int* bar = &F.ctrl->bar;
@@ -1565,15 +1579,15 @@ __device__ void app_front(AppFront<R>& F, int rank, int nr, const FactorParams& 
     set_slot(F, j & 1);
     const StepView v = step_view(F.ctrl);
     if (v.stop) break;
-    app_rows(F, v, rank, nr, sm.Bs, sm.slab, sm.spv, sm.scm, sm.srm, Ls);
+    app_rows(F, v, rank, nr, sm.Bs, sm.slab, sm.spv, sm.scm, sm.srm, stage);
     if (!sync()) break;
     const int q = app_accept(F, v, rank, thr, inv_u, &sm.q, sm.Bs, sm.spv, sm.scm, sm.srm);
     if (q < v.w) {
-      app_restore(F, v, rank, nr, q);
+      app_restore(F, v, rank, nr, q, sm.Bs, sm.spv);
       if (!sync()) break;
     }
     la = q == v.w && v.p + v.w < v.lim;
-    app_update(F, v, rank, nr, q, la, Ls, Ws, sm.ca, sm.cb, sm.cd, sm.Bs, sm.spv);
+    app_update(F, v, rank, nr, q, la, stage);
     if (la && rank == 0) {
       __syncthreads();
       app_advance(F, q);
@@ -1596,14 +1610,13 @@ __global__ void __launch_bounds__(kAppThreads) k_front_app(const std::int32_t* l
                                                            std::int32_t* pidx_out, FactorParams prm,
                                                            FactorCounters* cnt, std::int32_t* failed) {
   extern __shared__ __align__(16) unsigned char app_dyn[];
-  R* Ls = reinterpret_cast<R*>(app_dyn);
-  R* Ws = Ls + kKB * kUpdLd;
+  R* stage = reinterpret_cast<R*>(app_dyn);
   __shared__ AppSmem<R> sm;
   const SnDev d = sn[list[blockIdx.x]];
   AppFront<R> F = make_front(d, panels, cb, scratch, piv_out, pidx_out);
   app_init(F, 0, 1);
   __syncthreads();
-  app_front<false>(F, 0, 1, prm, cnt, failed, nullptr, sm, Ls, Ws);
+  app_front<false>(F, 0, 1, prm, cnt, failed, nullptr, sm, stage);
 }
 
 // Cooperative: the fronts of a level share the grid; front f owns CTAs [cta_start[f], cta_start[f+1])
@@ -1618,8 +1631,7 @@ __global__ void __launch_bounds__(kAppThreads) k_front_coop(const std::int32_t* 
   namespace cg = cooperative_groups;
   cg::grid_group grid = cg::this_grid();
   extern __shared__ __align__(16) unsigned char app_dyn[];
-  R* Ls = reinterpret_cast<R*>(app_dyn);
-  R* Ws = Ls + kKB * kUpdLd;
+  R* stage = reinterpret_cast<R*>(app_dyn);
   __shared__ AppSmem<R> sm;
   int fi = 0;
   while (fi + 1 < nfronts && cta_start[fi + 1] <= static_cast<int>(blockIdx.x)) ++fi;
@@ -1629,7 +1641,7 @@ __global__ void __launch_bounds__(kAppThreads) k_front_coop(const std::int32_t* 
   AppFront<R> F = make_front(d, panels, cb, scratch, piv_out, pidx_out);
   app_init(F, rank, nr);
   grid.sync();  // the control blocks (and their barrier counts) are initialized
-  app_front<true>(F, rank, nr, prm, cnt, failed, level_done, sm, Ls, Ws);
+  app_front<true>(F, rank, nr, prm, cnt, failed, level_done, sm, stage);
 }
 
 // ------------------------------------------------------------------------------ launchers

@@ -13,7 +13,9 @@ constexpr int kNB = 32;                // panel width of the a-posteriori pivoti
 constexpr int kTile = 64;              // trailing-update tile (rows = cols)
 constexpr int kKB = 128;               // pending pivots whose trailing update is applied at once (blocked step)
 constexpr int kUpdLd = kTile + 4;      // column stride of the staged update operands (conflict-free fragment reads)
-constexpr int kAppDynDoubles = 2 * kKB * kUpdLd;  // dynamic shared memory of the panel kernels
+constexpr int kUpdChunk = 32;          // pivots of a tile's operands staged at once
+constexpr int kUpdStages = 4;          // staged chunks (one computed, the others in flight)
+constexpr int kAppDynDoubles = kUpdStages * 2 * kUpdChunk * kUpdLd;  // dynamic shared memory of the panel kernels
 constexpr int kRowStage = kNB * kNB + 4 * kNB;   // panel row step: the block's L and the D^-1 coefficients
 constexpr int kRowChunk = (kAppDynDoubles - kRowStage) / kNB;  // rows staged at once by the panel row step
 constexpr int kAppThreads = 256;
@@ -21,11 +23,12 @@ constexpr int kCoopMinFront = 192;     // levels whose largest panel front is at
 constexpr int kColsPerThread = kTile * kTile / kAppThreads;  // 16
 constexpr int kExtendAddCols = 8;      // contribution-block columns per extend-add CTA
 // per-front scratch of the panel kernels (doubles): control block, two sets (alternate panels) of
-// block, original block, labels, pivot types and column maxima, backup of the panel's rows
+// block, original block, labels, pivot types and column maxima, backup of the panel's rows, W = L D
+// of the pending pivots (at most kKB, and at most the front's k)
 constexpr int kAppCtrlDoubles = 8;
 constexpr int kAppSlotDoubles = 2 * kNB * kNB + kNB / 2 + kNB / 8 + 2 * kNB;
-inline std::int64_t app_scratch_doubles(int m) {
-  return kAppCtrlDoubles + 2 * kAppSlotDoubles + static_cast<std::int64_t>(m) * kNB;
+inline std::int64_t app_scratch_doubles(int m, int k) {
+  return kAppCtrlDoubles + 2 * kAppSlotDoubles + static_cast<std::int64_t>(m) * (kNB + (k < kKB ? k : kKB));
 }
 
 void launch_fill(double* x, std::int64_t n, double v, cudaStream_t s);

@@ -387,7 +387,7 @@ std::shared_ptr<FrontPlan> GpuFactor::make_plan() {
       else {
         app.push_back(s);
         sn[s].scratch_off = scratch;
-        scratch += app_scratch_doubles(m);
+        scratch += app_scratch_doubles(m, k);
       }
     }
     scratch_max = std::max(scratch_max, scratch);
