@@ -989,62 +989,85 @@ __device__ void app_control_and_block(AppFront<R>& F, const FactorParams& prm, d
 }
 
 // All ranks: rows [p+w, m) solved against the block (L21 = F21 P L11^-T D^-1), backup, column maxima.
-// The block's strict lower part with the 2x2 couplings masked (they belong to D) is staged in Ls
-// (shared). The rows of a rank go through shared memory in chunks of kRowChunk: all threads load
-// the chunk (coalesced, batches of loads in flight at once) and write the backup; one thread per row
-// runs the substitution fully unrolled in registers and applies D^-1 through per-column coefficients
-// (no branch on the pivot type, every store after the last load); a warp per four columns then
-// writes the L values back (coalesced) and reduces the column maxima.
+// The rows of a rank go through shared memory in chunks of kRowChunk: the copies of the chunk are
+// issued before the block's arrays are read, four lanes run a row's substitution (lane q owns columns
+// q, q + 4, ..; a finished value goes to the other three by shuffle, every sum in the order of its
+// columns) and write the backup, and a warp per four columns applies D^-1 through per-column
+// coefficients (no branch on the pivot type), writes L and W = L D back (coalesced) and reduces the
+// column maxima. The phase is a chain of latencies (a rank of the n = 109,744 box's root holds at most
+// 45 rows): with one thread a row (496 dependent-load FMAs, 3.3 us) and the copies after the block it
+// took 7.9 us a panel, now 4.9.
 template <class R>
 __device__ void app_rows(AppFront<R>& F, const StepView& v, int rank, int nr, R* Bs, int* slab, signed char* spv,
-                         unsigned long long* scm, unsigned long long* srm, R* Lm) {
+                         R* Lm) {
   const int p = v.p, w = v.w, eb = v.eb, m = F.f.m;
-  for (int t = threadIdx.x; t < kNB * kNB; t += blockDim.x) Bs[t] = __ldcg(&F.B[t]);
-  for (int t = threadIdx.x; t < kNB; t += blockDim.x) {
-    slab[t] = __ldcg(&F.lab[t]);
-    spv[t] = __ldcg(&F.pv[t]);
-    scm[t] = 0ull;
-    srm[t] = 0ull;
-  }
-  __syncthreads();
-  // Lm[t * kNB + s] = L11(t, s) for s < min(t, eb), zero otherwise (row-major for broadcast reads)
-  for (int e = threadIdx.x; e < kNB * kNB; e += blockDim.x) {
-    const int t = e / kNB, s = e % kNB;
-    R x = R(0);
-    if (t < w && s < t && s < eb && !(spv[s] == 2 && s + 1 == t)) x = Bs[t + s * kNB];
-    Lm[e] = x;
-  }
-  // D^-1 as three coefficients per column: out(t) = k0 y(t-1) + k1 y(t) + k2 y(t+1); ksel says
-  // which value the column maximum takes: 0 |out|, 1 |y| (null pivot, l = 0), 2 none (t >= eb)
+  // D^-1 as three coefficients per column: l(t) = k0 y(t-1) + k1 y(t) + k2 y(t+1); ksel says
+  // which value the column maximum takes: 0 |l|, 1 |y| (null pivot, l = 0), 2 none (t >= eb)
   R* k0 = Lm + kNB * kNB;
   R* k1 = k0 + kNB;
   R* k2 = k1 + kNB;
   int* ksel = reinterpret_cast<int*>(k2 + kNB);
   R* Y = Lm + kRowStage;  // kNB columns of kRowChunk rows
-  for (int t = threadIdx.x; t < kNB; t += blockDim.x) {
+  const int rtotal = m - (p + w);
+  const int rchunk = (rtotal + nr - 1) / nr;
+  const int rbeg = p + w + rank * rchunk, rend = min(m, rbeg + rchunk);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // warp `warp` copies, writes back and reduces the maxima of columns 4 warp .. 4 warp + 3 (eight warps)
+  static_assert(kAppThreads / 32 * 4 == kNB, "a warp takes four columns");
+  auto stage = [&](int c0, int nrow) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int t = 4 * warp + c;
+      if (t >= w) break;
+      const R* col = F.f.panel + static_cast<std::int64_t>(p + t) * m + c0;
+      for (int r = lane; r < nrow; r += 32) cp_async_elem(&Y[t * kRowChunk + r], col + r, true);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  __syncthreads();  // the staging area's last users are done
+  if (rbeg < rend) stage(rbeg, min(kRowChunk, rend - rbeg));
+  // the block: Bs as it is; Lm(t, s) = L11(t, s) for s < min(t, eb), zero otherwise (2x2 couplings
+  // belong to D)
+#pragma unroll
+  for (int u = 0; u < kNB * kNB / kAppThreads; ++u) {
+    const int e = threadIdx.x + u * kAppThreads, t = e & (kNB - 1), s = e / kNB;
+    const R x = __ldcg(&F.B[e]);
+    const signed char ty = __ldcg(&F.pv[s]);
+    Bs[e] = x;
+    Lm[e] = t > s && t < w && s < eb && !(ty == 2 && t == s + 1) ? x : R(0);
+  }
+  bool moved = false;
+  if (threadIdx.x < kNB) {
+    const int t = threadIdx.x;
+    const signed char ty = __ldcg(&F.pv[t]);
+    const int from = __ldcg(&F.lab[t]);
+    const R* b = F.B;
     R a0 = R(0), a1 = R(1), a2 = R(0);
     int sel = 2;
     if (t < eb) {
-      const signed char ty = spv[t];
       sel = 0;
       if (ty == 0) { a1 = R(0); sel = 1; }
-      else if (ty == 1) a1 = R(1) / Bs[t + t * kNB];
+      else if (ty == 1) a1 = R(1) / __ldcg(&b[t + t * kNB]);
       else {
         const int f0 = ty == 2 ? t : t - 1;
-        const R a = Bs[f0 + f0 * kNB], b = Bs[f0 + 1 + f0 * kNB], cc = Bs[f0 + 1 + (f0 + 1) * kNB];
-        const R idet = R(1) / (a * cc - b * b);
+        const R a = __ldcg(&b[f0 + f0 * kNB]), c = __ldcg(&b[f0 + 1 + f0 * kNB]);
+        const R cc = __ldcg(&b[f0 + 1 + (f0 + 1) * kNB]);
+        const R idet = R(1) / (a * cc - c * c);
         // first of the pair: l = (c y_t - b y_{t+1}) / det; second: l = (a y_t - b y_{t-1}) / det
-        if (ty == 2) { a1 = cc * idet; a2 = -b * idet; }
-        else { a0 = -b * idet; a1 = a * idet; }
+        if (ty == 2) { a1 = cc * idet; a2 = -c * idet; }
+        else { a0 = -c * idet; a1 = a * idet; }
       }
     }
     k0[t] = a0;
     k1[t] = a1;
     k2[t] = a2;
     ksel[t] = sel;
+    slab[t] = from;
+    spv[t] = ty;
+    moved = t < w && from != t;
   }
   // did the block factorization swap any of its rows? (rarely: then the permutation below moves data)
-  const bool permuted = __syncthreads_or(threadIdx.x < w && slab[threadIdx.x] != static_cast<int>(threadIdx.x)) != 0;
+  const bool permuted = __syncthreads_or(moved) != 0;
   // permute the L rows p..p+w-1 of the eliminated columns c < p (a thread owns a column; the
   // columns are split into contiguous chunks over the ranks)
   const int cchunk = (p + nr - 1) / nr;
@@ -1058,94 +1081,72 @@ __device__ void app_rows(AppFront<R>& F, const StepView& v, int rank, int nr, R*
     for (int a = 0; a < kNB; ++a)
       if (a < w) colp[a] = x[a];
   }
-  const int rtotal = m - (p + w);
-  const int rchunk = (rtotal + nr - 1) / nr;
-  const int rbeg = p + w + rank * rchunk, rend = min(m, rbeg + rchunk);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // warp `warp` writes back and reduces the maxima of columns 4 warp .. 4 warp + 3 (eight warps)
-  static_assert(kAppThreads / 32 * 4 == kNB, "the write-back pass takes four columns per warp");
-  constexpr int kStageBatch = 8;
+  constexpr int kBatch = 4;
   // column maxima in FP32 (rounding is monotone: the maximum of the rounded values is the rounded
   // maximum), reduced over the warp with one integer max on the bit patterns of the non-negative floats
   float cm[4] = {0.0f, 0.0f, 0.0f, 0.0f};
   for (int c0 = rbeg; c0 < rend; c0 += kRowChunk) {
     const int nrow = min(kRowChunk, rend - c0);
-    const int total = w * nrow;
-    __syncthreads();
-    // stage: element e = (column t, row r), column-major, consecutive threads on consecutive rows;
-    // a batch of loads is issued before any store (the stores could alias later loads)
-    for (int e0 = threadIdx.x; e0 < total; e0 += kStageBatch * kAppThreads) {
-      R x[kStageBatch];
-#pragma unroll
-      for (int u = 0; u < kStageBatch; ++u) {
-        const int e = e0 + u * kAppThreads;
-        const int t = e / nrow, r = e - t * nrow;
-        x[u] = e < total ? F.f.at(c0 + r, p + slab[t]) : R(0);
-      }
-#pragma unroll
-      for (int u = 0; u < kStageBatch; ++u) {
-        const int e = e0 + u * kAppThreads;
-        if (e < total) {
-          const int t = e / nrow, r = e - t * nrow;
-          F.backup[static_cast<std::int64_t>(t) * m + c0 + r] = x[u];
-          Y[t * kRowChunk + r] = x[u];
-        }
-      }
+    if (c0 > rbeg) {
+      __syncthreads();
+      stage(c0, nrow);
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    // one thread per row: substitution and D^-1 in registers, then the row back to shared memory
-    // (the l values; |y| of a null pivot column, whose l is zero, for its maximum)
-    for (int r = threadIdx.x; r < nrow; r += kAppThreads) {
-      R y[kNB];
+    // four lanes per row, eight rows per warp; lanes without a row follow along for the shuffles
+    const int q = lane & 3;
+    for (int r0 = 0; r0 < nrow; r0 += kAppThreads / 4) {
+      const int r = r0 + (threadIdx.x >> 2);
+      const bool in = r < nrow;
+      if (r0 + 8 * warp >= nrow) break;
+      R y[kNB / 4];
 #pragma unroll
-      for (int t = 0; t < kNB; ++t) y[t] = t < w ? Y[t * kRowChunk + r] : R(0);
-#pragma unroll
-      for (int t = 1; t < kNB; ++t) {
-        R acc = y[t];
-#pragma unroll
-        for (int s2 = 0; s2 < t; ++s2) acc = fma(-y[s2], Lm[t * kNB + s2], acc);
-        y[t] = acc;
-      }
-      // the substituted row is W = L D, the update's second operand (zero for a null pivot)
-      R* wrow = F.wd + static_cast<std::int64_t>(p - v.fb) * m + c0 + r;
-#pragma unroll
-      for (int t = 0; t < kNB; ++t)
-        if (t < eb) wrow[static_cast<std::int64_t>(t) * m] = ksel[t] == 1 ? R(0) : y[t];
-      R prev = R(0);
-#pragma unroll
-      for (int t = 0; t < kNB; ++t) {
-        const R yn = t + 1 < kNB ? y[t + 1 < kNB ? t + 1 : t] : R(0);
-        const R out = fma(k0[t], prev, fma(k2[t], yn, k1[t] * y[t]));
-        prev = y[t];
-        y[t] = ksel[t] == 1 ? y[t] : out;
-        // the coefficients are read eight columns at a time (hoisting all of them would spill)
-        if ((t & 7) == 7) asm volatile("" ::: "memory");
+      for (int j = 0; j < kNB / 4; ++j) {
+        const int t = q + 4 * j;
+        y[j] = in && t < w ? Y[slab[t] * kRowChunk + r] : R(0);
+        if (in && t < w) F.backup[static_cast<std::int64_t>(t) * m + c0 + r] = y[j];
       }
 #pragma unroll
-      for (int t = 0; t < kNB; ++t)
-        if (t < w) Y[t * kRowChunk + r] = y[t];
+      for (int s = 0; s < kNB - 1; ++s) {
+        const R ys = __shfl_sync(0xffffffffu, y[s / 4], s & 3, 4);
+#pragma unroll
+        for (int j = s / 4; j < kNB / 4; ++j) y[j] = fma(-ys, Lm[s * kNB + q + 4 * j], y[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < kNB / 4; ++j)
+        if (in && q + 4 * j < w) Y[(q + 4 * j) * kRowChunk + r] = y[j];
     }
     __syncthreads();
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       const int t = 4 * warp + c;
-      if (t < w) {
-        const int sel = ksel[t];
-        R* colp = F.f.col(p + t) + c0;
-        // a batch of shared-memory reads before the global stores (which could alias them)
-        for (int r0 = lane; r0 < nrow; r0 += 32 * kStageBatch) {
-          R x[kStageBatch];
+      if (t >= w) break;
+      const int sel = ksel[t];
+      const R a0 = k0[t], a1 = k1[t], a2 = k2[t];
+      const bool two = a0 != R(0) || a2 != R(0);
+      const R* yt = Y + t * kRowChunk;
+      R* colp = F.f.panel + static_cast<std::int64_t>(p + t) * m + c0;
+      R* wcol = F.wd + static_cast<std::int64_t>(p - v.fb + t) * m + c0;
+      // a batch of shared-memory reads before the global stores (which could alias them)
+      for (int r0 = lane; r0 < nrow; r0 += 32 * kBatch) {
+        R x[kBatch], l[kBatch];
 #pragma unroll
-          for (int u = 0; u < kStageBatch; ++u) {
-            const int r = r0 + 32 * u;
-            x[u] = r < nrow ? Y[t * kRowChunk + r] : R(0);
-          }
+        for (int u = 0; u < kBatch; ++u) {
+          const int r = r0 + 32 * u;
+          x[u] = r < nrow ? yt[r] : R(0);
+          l[u] = a1 * x[u];
+          if (two && r < nrow)
+            l[u] = fma(a0, t > 0 ? yt[r - kRowChunk] : R(0), fma(a2, t + 1 < kNB ? yt[r + kRowChunk] : R(0), l[u]));
+        }
 #pragma unroll
-          for (int u = 0; u < kStageBatch; ++u) {
-            const int r = r0 + 32 * u;
-            if (r < nrow) colp[r] = sel == 1 ? R(0) : x[u];
-            if (sel != 2) cm[c] = fmaxf(cm[c], static_cast<float>(fabs(x[u])));
+        for (int u = 0; u < kBatch; ++u) {
+          const int r = r0 + 32 * u;
+          if (r < nrow) {
+            colp[r] = sel == 1 ? R(0) : l[u];
+            // the substituted row is W = L D, the update's second operand (zero for a null pivot)
+            if (sel != 2) wcol[r] = sel == 1 ? R(0) : x[u];
           }
+          if (sel != 2) cm[c] = fmaxf(cm[c], static_cast<float>(fabs(sel == 1 ? x[u] : l[u])));
         }
       }
     }
@@ -1163,8 +1164,6 @@ __device__ void app_rows(AppFront<R>& F, const StepView& v, int rank, int nr, R*
       atomicMax(&F.rmax[t], bits);
     }
   }
-  (void)scm;
-  (void)srm;
 }
 
 // All ranks: the accepted prefix q (identical in every CTA); rank 0 books the inertia. The small
@@ -1579,7 +1578,7 @@ __device__ void app_front(AppFront<R>& F, int rank, int nr, const FactorParams& 
     set_slot(F, j & 1);
     const StepView v = step_view(F.ctrl);
     if (v.stop) break;
-    app_rows(F, v, rank, nr, sm.Bs, sm.slab, sm.spv, sm.scm, sm.srm, stage);
+    app_rows(F, v, rank, nr, sm.Bs, sm.slab, sm.spv, stage);
     if (!sync()) break;
     const int q = app_accept(F, v, rank, thr, inv_u, &sm.q, sm.Bs, sm.spv, sm.scm, sm.srm);
     if (q < v.w) {
