@@ -390,98 +390,202 @@ __device__ void dense_bk_step(R* F, int ld, int m, int nfs, bool root, double u,
   __syncthreads();
 }
 
-// Warp maximum of non-negative floats: their bit patterns order like the values, so one integer
-// warp reduction replaces a shuffle tree.
-__device__ __forceinline__ float warp_maxf(float v) {
-  return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+__device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(d0), "+d"(d1) : "d"(a), "d"(b));
 }
 
-// Runs of plain 1x1 pivots, the common case, by the whole CTA: the lower triangle (order m <= MAXM)
-// is in registers, column c in warp c % NW (slot c / NW), row i in lane i % 32. From st.j on, every
-// warp reads the pivot column from shared memory, takes the same decision from it and updates its own
-// columns; the owner of the next column publishes it (two buffers, so one block barrier per pivot).
-// Ends at st.lim or at the first column whose 1x1 test fails (nothing of that column is changed). The
-// column maximum is reduced in FP32, rounded up, so a pivot that passes here passes the test in FP64.
-//
-// A pivot is a chain of dependent operations (column read, 1 / d beside the maximum, update, write,
-// barrier), not work: one warp alone needed 1,400 cycles per pivot for the same block, most of them for the
-// update of its 32 columns one after another (the look-ahead step of a root panel of the n = 109,744 box:
-// 24.3 us with one warp, 12.7 us with the CTA; a whole count at n = 737, fronts up to 109: 735 -> 579 us).
+// 1 / d for normal d away from the ends of the exponent range: the hardware's approximation and
+// Newton's iteration r += r (1 - d r). Without the range branches of a division, the pivot chain below
+// can be scheduled around it.
+__device__ __forceinline__ double rcp_newton(double d) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  double e = fma(-d, r, 1.0);
+  e = fma(e, e, e);
+  r = fma(e, r, r);
+  e = fma(-d, r, 1.0);
+  return fma(e, r, r);
+}
+__device__ __forceinline__ float rcp_newton(float d) { return 1.0f / d; }
+constexpr double kRcpMin = 1e-280, kRcpMax = 1e280;  // |d| that rcp_newton is used for
+
+// The bits of |v| that order like the values (the upper word of a double), and a bound of every
+// value with those bits.
+__device__ __forceinline__ unsigned mag_bits(double v) { return static_cast<unsigned>(__double2hiint(v)) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned mag_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+__device__ __forceinline__ double mag_upper(unsigned b, double) { return __hiloint2double(static_cast<int>(b) + 1, 0); }
+__device__ __forceinline__ double mag_upper(unsigned b, float) { return static_cast<double>(__uint_as_float(b)); }
+constexpr double kMagSlack = 1.0 + 4e-6;  // mag_upper is at most this factor above the value
+
+// The lower triangle of a matrix of order MAXM in the registers of NT threads, by 8 x 8 blocks dealt to
+// the warps in the layout of the FP64 tensor instruction's accumulator (lane: row lane / 4, columns
+// 2 (lane % 4), + 1 of the block).
 template <int MAXM, int NT, class R>
-__device__ __forceinline__ void fast_pivots(R (&y)[MAXM / (NT / 32)][MAXM / 32], R* buf, double u, double thr,
-                                            signed char* pv, StepShared& st) {
-  constexpr int NW = NT / 32, NC = MAXM / NW, NR = MAXM / 32;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+struct RegTri {
+  static constexpr int NW = NT / 32, NB8 = MAXM / 8, NBLK = NB8 * (NB8 + 1) / 2, PER = (NBLK + NW - 1) / NW;
+  static constexpr int kNone = 1 << 20;
+  R v[PER][2];
+  int r0[PER], c0[PER];  // this lane's row and first column of the warp's blocks (kNone: no block)
+  __device__ __forceinline__ void place() {
+    const int warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int s = 0; s < PER; ++s) {
+      int b = NW - 1 - warp + NW * s, bj = 0;
+      while (bj < NB8 && b >= NB8 - bj) { b -= NB8 - bj; ++bj; }
+      r0[s] = 8 * (bj + b) + ((threadIdx.x & 31) >> 2);
+      c0[s] = bj < NB8 ? 8 * bj + 2 * (threadIdx.x & 3) : kNone;
+    }
+  }
+  // f(value, row, column) for this lane's entries on or below the diagonal
+  template <class Fn>
+  __device__ __forceinline__ void each(Fn&& f) {
+#pragma unroll
+    for (int s = 0; s < PER; ++s)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        if (c0[s] != kNone && r0[s] >= c0[s] + e) f(v[s][e], r0[s], c0[s] + e);
+  }
+};
+
+// Shared memory of fast_pivots: four columns before their elimination, their L and W = L D (row-major).
+template <int MAXM, class R>
+struct __align__(16) QuadSmem {
+  R col[4 * MAXM + 16], l[4 * MAXM], x[4 * MAXM];
+  int npass;
+};
+
+// Runs of plain 1x1 pivots, the common case, by the whole CTA: the matrix is in registers (y; entries
+// of rows and columns beyond its order are zero), four pivots a step. The owners publish the four
+// columns; warp 0 (a row per lane, the 4 x 4 block's own elimination in every lane) eliminates them and
+// tests each: 1x1 against the largest entry below, rounded up, so a pivot that passes here passes the
+// exact test; every warp applies the pivots up to the first failure to its blocks (FP64: one tensor
+// instruction a block). The eliminated columns, L with D on the diagonal, go to F (order ld, shared).
+// Ends at st.lim or before the first column whose test fails.
+//
+// A pivot is a chain of dependent operations (1 / d, scale, update, the next d), not work. A 32 x 32
+// block takes 7,700 cycles; with one warp for the whole block it took 36,100, with one pivot a
+// barrier 12,800.
+template <int MAXM, int NT, class R>
+__device__ __forceinline__ void fast_pivots(RegTri<MAXM, NT, R>& y, QuadSmem<MAXM, R>& sm, R* F, int ld, double u,
+                                            double thr, signed char* pv, StepShared& st) {
+  constexpr int NR = MAXM / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t4 = lane & 3, g = lane >> 2;
   int j = st.j;
   const int lim = st.lim;
-  auto publish = [&](int c) {
-    if ((c & (NW - 1)) != warp) return;
-    const int slot = c / NW;
-    R v[NR];
+  const double nul = thr >= 0.0 ? thr * kMagSlack : -1.0;
+  int np = 4;
+  while (np == 4 && j < lim) {
 #pragma unroll
-    for (int r = 0; r < NR; ++r) v[r] = y[0][r];
+    for (int s = 0; s < y.PER; ++s)
 #pragma unroll
-    for (int s = 1; s < NC; ++s)
-      if (slot == s) {
+      for (int e = 0; e < 2; ++e) {
+        const int t = y.c0[s] + e - j;
+        if (static_cast<unsigned>(t) < 4u) sm.col[y.r0[s] * 4 + t] = y.v[s][e];
+      }
+    __syncthreads();
+    // (rows above j hold leftovers: they reach only entries above the diagonal or of eliminated columns)
+    R x[4][NR], l[4][NR];
+    if (warp == 0) {
+      R a[4][4];
 #pragma unroll
-        for (int r = 0; r < NR; ++r) v[r] = y[s][r];
+      for (int s = 0; s < 4; ++s)
+#pragma unroll
+        for (int t = 0; t <= s; ++t) a[t][s] = sm.col[(j + s) * 4 + t];
+#pragma unroll
+      for (int r = 0; r < NR; ++r)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) x[t][r] = sm.col[(lane + 32 * r) * 4 + t];
+      double gc[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const R inv = rcp_newton(a[t][t]);
+        R la[4];
+#pragma unroll
+        for (int s = t + 1; s < 4; ++s) la[s] = a[t][s] * inv;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) l[t][r] = x[t][r] * inv;
+#pragma unroll
+        for (int s2 = t + 1; s2 < 4; ++s2) {
+#pragma unroll
+          for (int s = s2; s < 4; ++s) a[s2][s] -= la[s] * a[t][s2];
+#pragma unroll
+          for (int r = 0; r < NR; ++r) x[s2][r] -= l[t][r] * a[t][s2];
+        }
+        unsigned gb = 0;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) gb = max(gb, lane + 32 * r > j + t ? mag_bits(x[t][r]) : 0u);
+        gc[t] = mag_upper(__reduce_max_sync(0xffffffffu, gb), a[0][0]);
       }
 #pragma unroll
-    for (int r = 0; r < NR; ++r) buf[(c & 1) * MAXM + lane + 32 * r] = v[r];
-  };
-  publish(j);
-  __syncthreads();
-  const int j0 = j;
-  int neg = 0;
-  const double nul = thr * (1.0 + 1e-6);
-  while (j < lim) {
-    const R* col = buf + (j & 1) * MAXM;
-    const R d = col[j];
-    R x[NR], yc[NC];
-    float g = 0.0f;
+      for (int r = 0; r < NR; ++r)
 #pragma unroll
-    for (int r = 0; r < NR; ++r) {
-      const int i = lane + 32 * r;
-      x[r] = i > j ? col[i] : R(0);
-      if constexpr (sizeof(R) == 8) g = fmaxf(g, __double2float_ru(fabs(x[r])));
-      else g = fmaxf(g, fabsf(x[r]));
+        for (int t = 0; t < 4; ++t) {
+          sm.l[(lane + 32 * r) * 4 + t] = l[t][r];
+          sm.x[(lane + 32 * r) * 4 + t] = x[t][r];
+        }
+      unsigned pass = 0, negs = 0;
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const double dcc = fabs(static_cast<double>(a[t][t]));
+        const bool ok = (j + t < lim) & (dcc >= kRcpMin) & (dcc <= kRcpMax) & (dcc >= u * gc[t]) &
+                        ((dcc > nul) | (gc[t] > nul));
+        pass |= ok ? 1u << t : 0u;
+        negs |= a[t][t] < R(0) ? 1u << t : 0u;
+      }
+      const int n = __ffs(~pass) - 1;
+      if (lane < n) pv[j + lane] = 1;
+      if (lane == 0) {
+        sm.npass = n;
+        const int neg = __popc(negs & ((1u << n) - 1u));
+        st.neg += neg;
+        st.pos += n - neg;
+      }
     }
+    __syncthreads();
+    np = sm.npass;
 #pragma unroll
-    for (int s = 0; s < NC; ++s) yc[s] = col[warp + NW * s];
-    const R inv = R(1) / d;
-    const double gc = warp_maxf(g);
-    const double dcc = fabs(static_cast<double>(d));
-    if (!(dcc > 0.0 && dcc >= u * gc) || (thr >= 0.0 && fmax(dcc, gc) <= nul)) break;
+    for (int s = 0; s < y.PER; ++s) {
+      const int rb = y.r0[s] - g, cb = y.c0[s] - 2 * t4;
+      if (y.c0[s] != y.kNone && cb + 7 > j) {
+        if constexpr (sizeof(R) == 8) {
+          const R a = sm.l[(rb + g) * 4 + t4], b = sm.x[(cb + g) * 4 + t4];
+          dmma_m8n8k4(y.v[s][0], y.v[s][1], t4 < np ? -a : R(0), t4 < np ? b : R(0));
+        } else {
 #pragma unroll
-    for (int r = 0; r < NR; ++r) x[r] *= inv;
+          for (int t = 0; t < 4; ++t) {
+            const R a = sm.l[(rb + g) * 4 + t];
 #pragma unroll
-    for (int s = 0; s < NC; ++s)
-      if (warp + NW * s > j) {
-#pragma unroll
-        for (int r = 0; r < NR; ++r) y[s][r] -= x[r] * yc[s];
+            for (int e = 0; e < 2; ++e) {
+              const R b = sm.x[(y.c0[s] + e) * 4 + t];
+              y.v[s][e] = t < np ? fma(-a, b, y.v[s][e]) : y.v[s][e];
+            }
+          }
+        }
       }
-    if (j + 1 < lim) publish(j + 1);
-    if ((j & (NW - 1)) == warp) {
+    }
+    if (warp == 0) {
 #pragma unroll
-      for (int s = 0; s < NC; ++s)
-        if (j / NW == s) {
+      for (int t = 0; t < 4; ++t)
 #pragma unroll
-          for (int r = 0; r < NR; ++r)
-            if (lane + 32 * r > j) y[s][r] = x[r];
+        for (int r = 0; r < NR; ++r) {
+          const int i = lane + 32 * r;
+          if (i >= j + t && i < ld && t < np) F[i + (j + t) * ld] = i == j + t ? x[t][r] : l[t][r];
         }
     }
-    if (threadIdx.x == 0) pv[j] = 1;
-    if (d < R(0)) ++neg;
-    ++j;
-    __syncthreads();
+    j += np;
   }
-  if (threadIdx.x == 0 && j > j0) {
-    st.neg += neg;
-    st.pos += j - j0 - neg;
+  if (threadIdx.x == 0 && j > st.j) {
     st.j = j;
     st.prog = 1;
   }
   __syncthreads();
+}
+
+// Warp maximum of non-negative floats: their bit patterns order like the values, so one integer
+// warp reduction replaces a shuffle tree.
+__device__ __forceinline__ float warp_maxf(float v) {
+  return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
 }
 
 // One warp: one elimination of threshold Bunch-Kaufman on the panel's diagonal block (order w <= 32,
@@ -635,30 +739,23 @@ __device__ __forceinline__ void bk_begin(StepShared& st, int lim) {
   st.neg = st.pos = st.zero = st.two = st.forced = 0;
 }
 
-// The panel's diagonal block by the whole CTA: y holds its lower triangle (row lane, columns
-// warp + 8 s); st was begun (and a block barrier passed) before. The factored block is left in F
-// (shared, ld kNB, lower triangle).
+// The panel's diagonal block by the whole CTA: y holds its lower triangle (zero from order w on); st was
+// begun (and a block barrier passed) before. The factored block is left in F (shared, ld kNB, lower
+// triangle).
 template <class R>
-__device__ void block_bk(R (&y)[4][1], R* F, R* buf, int w, bool root, double u, double thr, int* lab, signed char* pv,
-                         StepShared& st) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+__device__ void block_bk(RegTri<kNB, kAppThreads, R>& y, R* F, QuadSmem<kNB, R>& qs, int w, bool root, double u,
+                         double thr, int* lab, signed char* pv, StepShared& st) {
   while (true) {
-    if (!st.force && st.j < st.lim) fast_pivots<kNB, kAppThreads>(y, buf, u, thr, pv, st);
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const int c = warp + 8 * s;
-      if (lane >= c && lane < w) F[lane + c * kNB] = y[s][0];
-    }
+    if (!st.force && st.j < st.lim) fast_pivots<kNB, kAppThreads>(y, qs, F, kNB, u, thr, pv, st);
+    const int j = st.j;
+    if (j >= w) break;
+    y.each([&](R& v, int i, int c) { if (c >= j && i < w) F[i + c * kNB] = v; });
     __syncthreads();
-    if (st.j >= w) break;
-    if (warp == 0) warp_block_step(F, w, root, u, thr, lab, pv, st);
+    if (threadIdx.x < 32) warp_block_step(F, w, root, u, thr, lab, pv, st);
     __syncthreads();
     if (st.stop || st.j >= w) break;
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const int c = warp + 8 * s;
-      if (lane >= c && lane < w) y[s][0] = F[lane + c * kNB];
-    }
+    y.each([&](R& v, int i, int c) { if (i < w) v = F[i + c * kNB]; });
+    __syncthreads();  // every entry is read before F changes again
   }
 }
 
@@ -666,16 +763,16 @@ __device__ void block_bk(R (&y)[4][1], R* F, R* buf, int w, bool root, double u,
 
 // ---------------------------------------------------------------------- small fronts (smem)
 
-// A front in registers: column c in warp c % NW, row i in lane i % 32 (fast_pivots); shared memory holds
-// it only for the general pivot steps (2x2 pivots, swaps, null and forced pivots).
+// A front in registers (fast_pivots); shared memory holds its eliminated columns, and all of it for the
+// general pivot steps (2x2 pivots, swaps, null and forced pivots).
 template <int MAXM, int NT, class R>
 __global__ void __launch_bounds__(NT) k_front_small(const std::int32_t* list, const SnDev* sn, R* panels, R* cb,
                                                     signed char* piv_out, std::int32_t* pidx_out, FactorParams prm,
                                                     FactorCounters* cnt, std::int32_t* failed) {
-  constexpr int NW = NT / 32, NC = MAXM / NW, NR = MAXM / 32;
   extern __shared__ __align__(16) unsigned char small_dyn[];
   R* F = reinterpret_cast<R*>(small_dyn);
-  __shared__ R tmp0[MAXM], tmp1[MAXM], buf[2 * MAXM];
+  __shared__ R tmp0[MAXM], tmp1[MAXM];
+  __shared__ QuadSmem<MAXM, R> qs;
   __shared__ int lab[MAXM];
   __shared__ signed char pv[MAXM];
   __shared__ StepShared st;
@@ -684,37 +781,33 @@ __global__ void __launch_bounds__(NT) k_front_small(const std::int32_t* list, co
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   R* panel = panels + d.panel_off;
   R* cbb = cb + d.cb_off;
-  // the lower triangle's entries of this thread: f(entry, pointer in the front's storage, i, c)
-  R y[NC][NR];
-  auto each = [&](auto&& f) {
-#pragma unroll
-    for (int s = 0; s < NC; ++s) {
-      const int c = warp + NW * s;
-      R* col = c < k ? panel + static_cast<std::int64_t>(c) * m : cbb + static_cast<std::int64_t>(c - k) * (m - k) - k;
-#pragma unroll
-      for (int r = 0; r < NR; ++r) {
-        const int i = lane + 32 * r;
-        f(y[s][r], col, i, c, c < m && i >= c && i < m);
-      }
-    }
+  auto at = [&](int i, int c) -> R& {
+    return c < k ? panel[static_cast<std::int64_t>(c) * m + i] : cbb[static_cast<std::int64_t>(c - k) * (m - k) + (i - k)];
   };
-  each([&](R& v, const R* col, int i, int, bool in) { v = in ? col[i] : R(0); });
+  RegTri<MAXM, NT, R> y;
+  y.place();
+#pragma unroll
+  for (int s = 0; s < y.PER; ++s) y.v[s][0] = y.v[s][1] = R(0);
+  y.each([&](R& v, int i, int c) { if (i < m) v = at(i, c); });
   for (int t = threadIdx.x; t < m; t += NT) lab[t] = t;
   if (threadIdx.x == 0) bk_begin(st, k);
   __syncthreads();
   const double thr = null_threshold(prm);
   while (true) {
-    if (!st.force && st.j < st.lim) fast_pivots<MAXM, NT>(y, buf, prm.u, thr, pv, st);
-    if (st.j >= k) break;
-    each([&](R& v, const R*, int i, int c, bool in) { if (in) F[i + c * ld] = v; });
+    if (!st.force && st.j < st.lim) fast_pivots<MAXM, NT>(y, qs, F, ld, prm.u, thr, pv, st);
+    const int j = st.j;
+    if (j >= k) break;
+    y.each([&](R& v, int i, int c) { if (c >= j && i < m) F[i + c * ld] = v; });
     __syncthreads();
     dense_bk_step(F, ld, m, k, d.parent < 0, prm.u, thr, lab, pv, tmp0, tmp1, st);
-    each([&](R& v, const R*, int i, int c, bool in) { if (in) v = F[i + c * ld]; });
+    y.each([&](R& v, int i, int c) { if (i < m) v = F[i + c * ld]; });
     if (st.stop) break;
-    __syncthreads();  // every column is read before a later step writes the matrix again
+    __syncthreads();  // every entry is read before F changes again
   }
   const int e = st.j;
-  each([&](const R& v, R* col, int i, int, bool in) { if (in) col[i] = v; });
+  for (int c = warp; c < e; c += NT / 32)
+    for (int i = c + lane; i < m; i += 32) panel[static_cast<std::int64_t>(c) * m + i] = F[i + c * ld];
+  y.each([&](R& v, int i, int c) { if (c >= e && i < m) at(i, c) = v; });
   for (int t = threadIdx.x; t < k; t += blockDim.x) {
     pidx_out[d.first + t] = lab[t];
     piv_out[d.first + t] = t < e ? pv[t] : static_cast<signed char>(-1);
@@ -869,7 +962,7 @@ __device__ void app_init(AppFront<R>& F, int rank, int nr) {
 // Rank 0: decide what the next panel is (stop = 1: front finished), and factorize its diagonal block
 // with block-restricted threshold Bunch-Kaufman; permute the L rows of the block; publish to scratch.
 template <class R>
-__device__ void app_control_and_block(AppFront<R>& F, const FactorParams& prm, double thr, R* Bs, R* tmp,
+__device__ void app_control_and_block(AppFront<R>& F, const FactorParams& prm, double thr, R* Bs, QuadSmem<kNB, R>& qs,
                                       int* slab, signed char* spv, StepShared& bst, int* shared_stop,
                                       FactorCounters* cnt, std::int32_t* failed, int* level_done) {
   AppCtrl* c = F.ctrl;
@@ -949,22 +1042,16 @@ __device__ void app_control_and_block(AppFront<R>& F, const FactorParams& prm, d
     __syncthreads();
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  R y[4][1];
+  RegTri<kNB, kAppThreads, R> y;
+  y.place();
 #pragma unroll
-  for (int s = 0; s < 4; ++s) {
-    const int c2 = warp + 8 * s;
-    const bool in = lane >= c2 && lane < w;
-    y[s][0] = in ? F.f.at(p + lane, p + c2) : R(0);
-  }
-#pragma unroll
-  for (int s = 0; s < 4; ++s) {
-    const int c2 = warp + 8 * s;
-    if (lane >= c2 && lane < w) F.Borig[lane + c2 * kNB] = y[s][0];
-  }
+  for (int s = 0; s < y.PER; ++s) y.v[s][0] = y.v[s][1] = R(0);
+  y.each([&](R& v, int i, int c2) { if (i < w) v = F.f.at(p + i, p + c2); });
+  y.each([&](R& v, int i, int c2) { if (i < w) F.Borig[i + c2 * kNB] = v; });
   for (int t = threadIdx.x; t < w; t += blockDim.x) slab[t] = t;
   if (threadIdx.x == 0) bk_begin(bst, w);
   __syncthreads();
-  block_bk(y, Bs, tmp, w, force, prm.u, thr, slab, spv, bst);
+  block_bk(y, Bs, qs, w, force, prm.u, thr, slab, spv, bst);
   const int eb = bst.j;
   if (__syncthreads_or(threadIdx.x < w && slab[threadIdx.x] != static_cast<int>(threadIdx.x))) {
     // the block's rows were swapped: its pivot labels follow
@@ -996,7 +1083,7 @@ __device__ void app_control_and_block(AppFront<R>& F, const FactorParams& prm, d
 // coefficients (no branch on the pivot type), writes L and W = L D back (coalesced) and reduces the
 // column maxima. The phase is a chain of latencies (a rank of the n = 109,744 box's root holds at most
 // 45 rows): with one thread a row (496 dependent-load FMAs, 3.3 us) and the copies after the block it
-// took 7.9 us a panel, now 4.9.
+// took 7.9 us a panel, now 5.3.
 template <class R>
 __device__ void app_rows(AppFront<R>& F, const StepView& v, int rank, int nr, R* Bs, int* slab, signed char* spv,
                          R* Lm) {
@@ -1269,11 +1356,6 @@ __device__ void app_restore(AppFront<R>& F, const StepView& v, int rank, int nr,
   }
 }
 
-__device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(d0), "+d"(d1) : "d"(a), "d"(b));
-}
-
 // Blocked step. The pivots [fb, p + q) eliminated since the last full update are pending: their
 // Schur update has reached only the panels factorized since. After a panel the pending update goes
 // either to the whole trailing matrix (a flush: the panel rejected columns, the candidate range
@@ -1495,7 +1577,7 @@ __device__ void app_advance(AppFront<R>& F, int q) {
 template <class R>
 struct AppSmem {
   R Bs[kNB * kNB];
-  R tmp[2 * kNB];
+  QuadSmem<kNB, R> qs;
   int slab[kNB];
   signed char spv[kNB];
   unsigned long long scm[kNB], srm[kNB];
@@ -1570,7 +1652,7 @@ __device__ void app_front(AppFront<R>& F, int rank, int nr, const FactorParams& 
       if (rank == 0) {
         if (j > 0) app_advance(F, qprev);
         set_slot(F, j & 1);
-        app_control_and_block(F, prm, thr, sm.Bs, sm.tmp, sm.slab, sm.spv, sm.bst, &sm.stop, cnt, failed,
+        app_control_and_block(F, prm, thr, sm.Bs, sm.qs, sm.slab, sm.spv, sm.bst, &sm.stop, cnt, failed,
                               level_done);
       }
       if (!sync()) break;
@@ -1591,7 +1673,7 @@ __device__ void app_front(AppFront<R>& F, int rank, int nr, const FactorParams& 
       __syncthreads();
       app_advance(F, q);
       set_slot(F, (j + 1) & 1);
-      app_control_and_block(F, prm, thr, sm.Bs, sm.tmp, sm.slab, sm.spv, sm.bst, &sm.stop, cnt, failed,
+      app_control_and_block(F, prm, thr, sm.Bs, sm.qs, sm.slab, sm.spv, sm.bst, &sm.stop, cnt, failed,
                             level_done);
     }
     if (!sync()) break;
