@@ -332,16 +332,14 @@ __device__ void dense_bk_step(R* F, int ld, int m, int nfs, bool root, double u,
   while (true) {
     if (threadIdx.x == 0) {
       st.stop = 0;
-      if (st.j >= nfs) st.stop = 1;
-      else if (st.j >= st.lim) {
-        if (st.prog) { st.lim = nfs; st.prog = 0; st.stop = 2; }
-        else if (root && !st.force) { st.force = 1; st.lim = nfs; st.stop = 2; }
-        else st.stop = 1;
+      while (st.j >= st.lim) {
+        if (st.j < nfs && st.prog) { st.lim = nfs; st.prog = 0; }
+        else if (st.j < nfs && root && !st.force) { st.force = 1; st.lim = nfs; }
+        else { st.stop = 1; break; }
       }
     }
     __syncthreads();
-    if (st.stop == 1) break;
-    if (st.stop == 2) continue;
+    if (st.stop) break;
     const int j = st.j;
     if (threadIdx.x < 32) decide_pivot(F, ld, m, nfs, j, u, thr, st.force != 0, st);
     __syncthreads();
@@ -623,8 +621,9 @@ __device__ __noinline__ void warp_block_step(R* F, int w, bool root, double u, d
     else if (dcc > 0.0 && dcc >= u * gc) dec = kOneJ;
     else {
       // partner candidate: argmax over rows (j, w) of |F(i, j)|
-      float best = lane > j && lane < w ? static_cast<float>(fabs(xj)) : -1.0f;
-      int bi = lane > j && lane < w ? lane : -1;
+      // (not a number counts as no candidate: the lanes have to agree on the partner)
+      float best = lane > j && lane < w && xj == xj ? static_cast<float>(fabs(xj)) : -1.0f;
+      int bi = best >= 0.0f ? lane : -1;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         const float ob = __shfl_xor_sync(0xffffffffu, best, o);
@@ -732,6 +731,8 @@ __device__ __noinline__ void warp_block_step(R* F, int w, bool root, double u, d
     st.neg += neg; st.pos += pos; st.zero += zero; st.two += two; st.forced += forced;
     st.j = j; st.lim = lim; st.prog = prog; st.force = force; st.stop = stop;
   }
+  // the lanes return together: the caller's block barrier counts the warp once, whichever lanes arrive
+  __syncwarp();
 }
 
 __device__ __forceinline__ void bk_begin(StepShared& st, int lim) {
@@ -1210,7 +1211,7 @@ __device__ void app_rows(AppFront<R>& F, const StepView& v, int rank, int nr, R*
       if (t >= w) break;
       const int sel = ksel[t];
       const R a0 = k0[t], a1 = k1[t], a2 = k2[t];
-      const bool two = a0 != R(0) || a2 != R(0);
+      const bool first = a0 != R(0), second = a2 != R(0);
       const R* yt = Y + t * kRowChunk;
       R* colp = F.f.panel + static_cast<std::int64_t>(p + t) * m + c0;
       R* wcol = F.wd + static_cast<std::int64_t>(p - v.fb + t) * m + c0;
@@ -1222,8 +1223,9 @@ __device__ void app_rows(AppFront<R>& F, const StepView& v, int rank, int nr, R*
           const int r = r0 + 32 * u;
           x[u] = r < nrow ? yt[r] : R(0);
           l[u] = a1 * x[u];
-          if (two && r < nrow)
-            l[u] = fma(a0, t > 0 ? yt[r - kRowChunk] : R(0), fma(a2, t + 1 < kNB ? yt[r + kRowChunk] : R(0), l[u]));
+          // (only the pair's own column is read: its neighbours may lie outside the panel)
+          if (second && r < nrow) l[u] = fma(a2, yt[r + kRowChunk], l[u]);
+          if (first && r < nrow) l[u] = fma(a0, yt[r - kRowChunk], l[u]);
         }
 #pragma unroll
         for (int u = 0; u < kBatch; ++u) {
