@@ -363,7 +363,7 @@ std::shared_ptr<FrontPlan> GpuFactor::make_plan() {
   std::int32_t hcnt_total = 0;  // backward helper counters: one per 32-column chunk of every front
   std::int64_t work_max = 0;
   std::vector<int2> sbl;
-  std::vector<int4> tiles;
+  std::vector<int4> tiles, narrow;
   std::int64_t w_total = 0;
   std::vector<std::int32_t> cptr;
   std::vector<ContribEntry> cent;
@@ -445,8 +445,16 @@ std::shared_ptr<FrontPlan> GpuFactor::make_plan() {
         dw.w_off = w_total;
         w_total += static_cast<std::int64_t>(dw.m) * dw.k;
         for (int b = 0, qb = 0; b < dw.k; b += kSB, ++qb) {
-          sbl.push_back(make_int2(sq, qb));
           const int be = std::min(b + kSB, dw.k);
+          if (be - b <= kSbNarrow) {
+            int r0 = be;
+            do {
+              narrow.push_back(make_int4(sq, qb, r0, r0 == be));
+              r0 += kNarrowRows;
+            } while (r0 < dw.m);
+            continue;
+          }
+          sbl.push_back(make_int2(sq, qb));
           for (int r0 = be; r0 < dw.m; r0 += 64) tiles.push_back(make_int4(sq, qb, r0, 0));
         }
       }
@@ -637,6 +645,8 @@ std::shared_ptr<FrontPlan> GpuFactor::make_plan() {
   P.cent.upload(cent, stream_);
   P.sbl.upload(sbl, stream_);
   P.tiles.upload(tiles, stream_);
+  P.narrow.upload(narrow, stream_);
+  P.nnarrow = static_cast<int>(narrow.size());
   P.nsbl = static_cast<int>(sbl.size());
   P.ntiles = static_cast<int>(tiles.size());
   P.scratch_max = scratch_max;
@@ -1000,7 +1010,9 @@ void GpuFactor::build_solve_operator() {
 
 template <class F>
 void GpuFactor::build_solve_operator_t() {
-  launch_sb_build<F>(plan_->sbl.p, plan_->nsbl, plan_->tiles.p, plan_->ntiles, plan_->sn.p, panels_of<F>(), d_piv_.p, w_of<F>(), stream_);
+  const FrontPlan& P = *plan_;
+  const SbLists lists{P.sbl.p, P.nsbl, P.tiles.p, P.ntiles, P.narrow.p, P.nnarrow};
+  launch_sb_build<F>(lists, P.sn.p, panels_of<F>(), d_piv_.p, w_of<F>(), stream_);
 }
 
 void GpuFactor::release() {

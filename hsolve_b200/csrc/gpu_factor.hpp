@@ -114,7 +114,7 @@ struct FrontPlan {
   std::int64_t vec_total = 0;      // contribution-vector rows of a solve
   std::int64_t arena_entries = 1;  // inertia-only counts: the largest level's panels
   std::int64_t scratch_max = 0, work_max = 0, w_total = 0;
-  int ncoop = 0, nsbl = 0, ntiles = 0;
+  int ncoop = 0, nsbl = 0, ntiles = 0, nnarrow = 0;
   std::int32_t hcnt_total = 0;     // backward helper counters (one per 32-column chunk of every front)
   DevBuf<std::int32_t> row, col;   // the union pattern's entries (row, column)
   DevBuf<std::int64_t> dest;       // their positions in the factor storage
@@ -129,8 +129,8 @@ struct FrontPlan {
   DevBuf<std::int32_t> pfirst;     // per pivot: first column of its front
   DevBuf<std::int32_t> cptr;       // children's contributions per front position
   DevBuf<ContribEntry> cent;
-  DevBuf<int2> sbl;                // super-blocks of the solve operators
-  DevBuf<int4> tiles;
+  DevBuf<int2> sbl;                // wide super-blocks of the solve operators
+  DevBuf<int4> tiles, narrow;
 };
 
 class GpuFactor {

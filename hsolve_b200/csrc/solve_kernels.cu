@@ -82,99 +82,253 @@ __global__ void k_solve_diag_flat(std::int64_t npiv, const std::int64_t* dpos, c
   }
 }
 
-// W[B, B] = L_BB^{-1} for one super-block per CTA: row-by-row substitution X[i, c] =
-// -sum_{c <= j < i} L[i, j] X[j, c] on packed triangles in shared memory (two threads per column).
+namespace {
+
+__device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
+}
+
+// factor entry to a double in shared memory (zero where not valid): asynchronously for FP64 factors
+__device__ __forceinline__ void stage_entry(double* dst, const double* src, bool valid) {
+  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(valid ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void stage_entry(double* dst, const float* src, bool valid) {
+  *dst = valid ? static_cast<double>(*src) : 0.0;
+}
+template <int N>
+__device__ __forceinline__ void stage_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void stage_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+
+// One warp: x <- L^{-1} x for a unit lower triangle L of order 32 and 32 right-hand sides, one per lane in
+// registers, every pivot's multiples subtracted from all later rows at once (independent FMAs).
+// L(i, j), i > j, at L[j * ldl + i].
+__device__ __forceinline__ void warp_unit_solve(const double* L, int ldl, double (&x)[32]) {
+#pragma unroll
+  for (int j = 0; j < 31; ++j)
+#pragma unroll
+    for (int i = j + 1; i < 32; ++i) x[i] = fma(-L[j * ldl + i], x[j], x[i]);
+}
+
+// Column strides of the staged operands: 4 (mod 16) doubles, so that every fragment read of the tensor
+// instructions hits 32 distinct banks per half-warp.
+constexpr int kRowsLd = 68;                // 64 rows of L, a column per pivot
+constexpr int kXLd = 36;                   // 32 pivots of X, a column per column
+constexpr int kInvLd = 132;                // a super-block
+constexpr std::size_t kInvSmem = sizeof(double) * (kSB * kInvLd + (kSB - 32) * kXLd);
+constexpr std::size_t kApplySmem = sizeof(double) * 2 * (32 * kRowsLd + kSB * kXLd);
+
+}  // namespace
+
+// Super-blocks of at most 32 pivots: the inverse (one warp) and its product with up to kNarrowRows rows
+// below it in one CTA. item: front, super-block, first row, 1 where the CTA also writes the inverse.
+// These are most super-blocks of a tree (the leaves' fronts), so what counts is their latency: the rows
+// of the first tile arrive while the triangle is inverted.
+template <class F>
+__global__ void __launch_bounds__(256) k_sb_narrow(const int4* items, const SnDev* sn, const F* panels,
+                                                   const signed char* piv, F* W) {
+  __shared__ double Xs[32 * kXLd], Ls[2][32 * kRowsLd];
+  double* Lb = Ls[1];  // the triangle, until the second tile is staged
+  const int4 e = items[blockIdx.x];
+  const SnDev d = sn[e.x];
+  const int m = d.m, b = e.y * kSB, bs = d.k - b, r0 = e.z;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
+  const F* P = panels + d.panel_off + static_cast<std::int64_t>(b) * m;
+  const signed char* pv = piv + d.first + b;
+  F* Wf = W + d.w_off + static_cast<std::int64_t>(b) * m;
+  const int rend = min(m, r0 + kNarrowRows);
+  const int ntile = (rend - r0 + 63) / 64;
+  // rows of a tile: warps over pivots, lanes over rows (pivots beyond bs are zero). A 2x2 pivot's
+  // coupling is D, not L: inside the block and where the block's end splits the pair.
+  auto stage = [&](int t) {
+    double* dst = Ls[t & 1];
+    for (int j = warp; j < 32; j += 8) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int row = lane + 32 * h, i = r0 + 64 * t + row;
+        const bool in = i < rend && j < bs && !(i == b + j + 1 && pv[j] == 2);
+        stage_entry(&dst[j * kRowsLd + row], in ? P + static_cast<std::int64_t>(j) * m + i : P, in);
+      }
+    }
+    stage_commit();
+  };
+  for (int j = warp; j < 32; j += 8) {
+    const bool in = lane > j && lane < bs && !(lane == j + 1 && pv[j] == 2);
+    Lb[j * 32 + lane] = in ? static_cast<double>(P[static_cast<std::int64_t>(j) * m + b + lane]) : 0.0;
+  }
+  if (ntile > 0) stage(0);
+  __syncthreads();
+  if (warp == 0) {
+    double x[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) x[i] = i == lane ? 1.0 : 0.0;
+    warp_unit_solve(Lb, 32, x);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) Xs[lane * kXLd + i] = x[i];
+  }
+  __syncthreads();
+  if (e.w)
+    for (int c = warp; c < bs; c += 8)
+      if (lane < bs) Wf[static_cast<std::int64_t>(c) * m + b + lane] = static_cast<F>(Xs[c * kXLd + lane]);
+  for (int t = 0; t < ntile; ++t) {
+    if (t + 1 < ntile) stage(t + 1);
+    else stage_commit();
+    stage_wait<1>();
+    __syncthreads();
+    const double* L = Ls[t & 1];
+    double acc[4][2] = {};
+#pragma unroll
+    for (int s0 = 0; s0 < 32; s0 += 4) {
+      if (s0 >= bs) break;
+      const double a = L[(s0 + t4) * kRowsLd + 8 * warp + g];
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (8 * q <= s0 + 3) dmma_8x8x4(acc[q], a, Xs[(8 * q + g) * kXLd + s0 + t4]);
+    }
+    const int i = r0 + 64 * t + 8 * warp + g;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int c = 8 * q + 2 * t4 + h;
+        if (i < rend && c < bs) Wf[static_cast<std::int64_t>(c) * m + i] = static_cast<F>(acc[q][h]);
+      }
+    __syncthreads();
+  }
+}
+
+// W[B, B] = L_BB^{-1} of a super-block of more than 32 pivots, in place in shared memory by block rows of
+// 32: T_ic = sum_j L_ij X_jc with the FP64 tensor instruction, then L_ii X_ic = -T_ic (and L_ii X_ii = I)
+// by substitution, a warp per 32 columns, a column per lane. (X_ic as the product of X_ii and T_ic
+// instead loses half a digit: errors of the solutions twice as large.) Row-by-row substitution by the
+// whole CTA, 128 dependent rows with two block barriers each, took 0.93 ms for the n = 109,744 box and
+// 0.34 ms for n = 3,021.
 template <class F>
 __global__ void __launch_bounds__(256) k_sb_inverse(const int2* sbl, const SnDev* sn, const F* panels,
                                                      const signed char* piv, F* W) {
   extern __shared__ double sm[];
-  double* Lp = sm;                                // strictly lower rows, row i at i(i-1)/2
-  double* Xp = sm + kSB * (kSB - 1) / 2;          // lower rows incl. diagonal, row i at i(i+1)/2
-  double* part = Xp + kSB * (kSB + 1) / 2;        // second-half partial sums
+  double* S = sm;                     // entry (i, j) at j * kInvLd + i
+  double* T = sm + kSB * kInvLd;      // entry (i, c) of the block row at c * kXLd + i
   const int2 e = sbl[blockIdx.x];
   const SnDev d = sn[e.x];
-  const int m = d.m;
-  const int b = e.y * kSB, bs = min(kSB, d.k - b);
-  const F* P = panels + d.panel_off;
-  const signed char* pv = piv + d.first;
-  for (int idx = threadIdx.x; idx < bs * bs; idx += blockDim.x) {
-    const int j = idx / bs, i = idx % bs;
-    if (i > j) Lp[i * (i - 1) / 2 + j] = (j + 1 == i && pv[b + j] == 2) ? 0.0 : P[(b + i) + static_cast<std::int64_t>(b + j) * m];
-  }
+  const int m = d.m, b = e.y * kSB, bs = min(kSB, d.k - b);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
+  const F* P = panels + d.panel_off + static_cast<std::int64_t>(b) * m + b;
+  const signed char* pv = piv + d.first + b;
+  const int order = (bs + 31) & ~31;
+  for (int j = warp; j < order; j += 8)
+    for (int i = lane; i < order; i += 32) {
+      const bool in = i > j && i < bs && !(i == j + 1 && pv[j] == 2);
+      stage_entry(&S[j * kInvLd + i], in ? P + static_cast<std::int64_t>(j) * m + i : P, in);
+    }
+  stage_commit();
+  stage_wait<0>();
   __syncthreads();
-  const int c = threadIdx.x & (kSB - 1), h = threadIdx.x / kSB;
-  for (int i = 0; i < bs; ++i) {
-    double acc = 0.0;
-    const double* Li = Lp + i * (i - 1) / 2;
-    for (int j = h; j < i; j += 2)
-      if (j >= c) acc = fma(Li[j], Xp[j * (j + 1) / 2 + c], acc);
-    if (h == 1) part[c] = acc;
+  for (int o = 0; o < order; o += 32) {
+    // T: warp w takes 8 rows and every other block of 8 columns
+    const int r = 8 * (warp & 3), h = warp >> 2;
+    double acc[6][2] = {};
+    for (int s0 = 0; s0 < o; s0 += 4) {
+      const double a = S[(s0 + t4) * kInvLd + o + r + g];
+#pragma unroll
+      for (int u = 0; u < 6; ++u) {
+        const int q = 2 * u + h;
+        if (8 * q <= s0 + 3 && 8 * q < o) dmma_8x8x4(acc[u], a, S[(8 * q + g) * kInvLd + s0 + t4]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 6; ++u)
+#pragma unroll
+      for (int z = 0; z < 2; ++z) {
+        const int c = 8 * (2 * u + h) + 2 * t4 + z;
+        if (c < o) T[c * kXLd + r + g] = acc[u][z];
+      }
     __syncthreads();
-    if (h == 0 && c <= i) Xp[i * (i + 1) / 2 + c] = c == i ? 1.0 : -(acc + part[c]);
+    double x[32];
+    const bool mine = 32 * warp <= o;
+    if (mine) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) x[i] = 32 * warp < o ? -T[(32 * warp + lane) * kXLd + i] : (i == lane ? 1.0 : 0.0);
+      warp_unit_solve(S + o * kInvLd + o, kInvLd, x);
+    }
+    __syncthreads();
+    if (mine)
+#pragma unroll
+      for (int i = 0; i < 32; ++i) S[(32 * warp + lane) * kInvLd + o + i] = x[i];
     __syncthreads();
   }
   F* Wd = W + d.w_off + b + static_cast<std::int64_t>(b) * m;
-  for (int idx = threadIdx.x; idx < bs * bs; idx += blockDim.x) {
-    const int cc = idx / bs, i = idx % bs;
-    Wd[i + static_cast<std::int64_t>(cc) * m] = static_cast<F>(i >= cc ? Xp[i * (i + 1) / 2 + cc] : 0.0);
-  }
+  for (int c = warp; c < bs; c += 8)
+    for (int i = lane; i < bs; i += 32)
+      Wd[i + static_cast<std::int64_t>(c) * m] = static_cast<F>(i >= c ? S[c * kInvLd + i] : 0.0);
 }
 
-// W[r0 : r0 + 64, B] = L[r0 : r0 + 64, B] W[B, B] for one 64-row tile below a super-block per CTA.
+// W[r0 : r0 + 64, B] = L[r0 : r0 + 64, B] W[B, B] for one 64-row tile below a super-block of more than 32
+// pivots per CTA, 32 pivots at a time (the next chunk in flight); a warp takes 8 rows and all columns,
+// pivots below a column (zero in W[B, B]) left out. On FMA units, with the zeros multiplied, the tiles of
+// the n = 109,744 box took 1.21 ms, now 0.43.
 template <class F>
-__global__ void __launch_bounds__(256) k_sb_apply(const int4* tiles, const SnDev* sn, const F* panels,
-                                                   const signed char* piv, F* W) {
-  __shared__ double Ls[32][64];
-  __shared__ double Xs[32][kSB];
+__global__ void __launch_bounds__(256, 2) k_sb_apply(const int4* tiles, const SnDev* sn, const F* panels,
+                                                      const signed char* piv, F* W) {
+  extern __shared__ double sm[];
   const int4 e = tiles[blockIdx.x];
   const SnDev d = sn[e.x];
   const int m = d.m;
   const int b = e.y * kSB, bs = min(kSB, d.k - b), r0 = e.z;
-  const F* P = panels + d.panel_off;
-  const signed char* pv = piv + d.first;
-  F* Wf = W + d.w_off;
-  const int tr = threadIdx.x & 15, tc = threadIdx.x >> 4;  // rows tr + 16 q, columns tc * 8 + p
-  double acc[4][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
+  const F* P = panels + d.panel_off + static_cast<std::int64_t>(b) * m;
+  const signed char* pv = piv + d.first + b;
+  F* Wf = W + d.w_off + static_cast<std::int64_t>(b) * m;
+  constexpr int kStage = 32 * kRowsLd + kSB * kXLd;
+  auto stage = [&](int j0, int st) {
+    double* Ls = sm + st * kStage;
+    double* Xs = Ls + 32 * kRowsLd;
+    for (int jj = warp; jj < 32; jj += 8) {
+      const int j = j0 + jj;
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
-#pragma unroll
-    for (int p = 0; p < 8; ++p) acc[q][p] = 0.0;
-  for (int j0 = 0; j0 < bs; j0 += 32) {
-    for (int idx = threadIdx.x; idx < 32 * 64; idx += blockDim.x) {
-      const int jj = idx / 64, row = idx % 64, i = r0 + row, j = j0 + jj;
-      // a 2 x 2 pivot split by the super-block boundary: its coupling entry is D, not L
-      const bool coupling = i == b + j + 1 && pv[b + j] == 2;
-      Ls[jj][row] = (i < m && j < bs && !coupling) ? P[i + static_cast<std::int64_t>(b + j) * m] : 0.0;
+      for (int h = 0; h < 2; ++h) {
+        const int row = lane + 32 * h, i = r0 + row;
+        // a 2 x 2 pivot split by the super-block boundary: its coupling entry is D, not L
+        const bool in = i < m && j < bs && !(i == b + j + 1 && pv[j] == 2);
+        stage_entry(&Ls[jj * kRowsLd + row], in ? P + static_cast<std::int64_t>(j) * m + i : P, in);
+      }
     }
-    for (int idx = threadIdx.x; idx < 32 * kSB; idx += blockDim.x) {
-      const int cc = idx / 32, jj = idx % 32, j = j0 + jj;
-      Xs[jj][cc] = (j < bs && cc < bs) ? Wf[(b + j) + static_cast<std::int64_t>(b + cc) * m] : 0.0;
+    for (int c = warp; c < min(bs, j0 + 32); c += 8) {
+      const bool in = j0 + lane < bs;
+      stage_entry(&Xs[c * kXLd + lane], in ? Wf + static_cast<std::int64_t>(c) * m + b + j0 + lane : Wf, in);
     }
+    stage_commit();
+  };
+  double acc[kSB / 8][2] = {};
+  stage(0, 0);
+  for (int j0 = 0, st = 0; j0 < bs; j0 += 32, st ^= 1) {
+    if (j0 + 32 < bs) stage(j0 + 32, st ^ 1);
+    else stage_commit();
+    stage_wait<1>();
     __syncthreads();
-#pragma unroll 4
-    for (int jj = 0; jj < 32; ++jj) {
-      double a[4], x[8];
+    const double* Ls = sm + st * kStage;
+    const double* Xs = Ls + 32 * kRowsLd;
+#pragma unroll 1
+    for (int s0 = 0; s0 < 32; s0 += 4) {
+      const double a = Ls[(s0 + t4) * kRowsLd + 8 * warp + g];
+      const int nq = min((j0 + s0) / 8 + 1, (bs + 7) / 8);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) a[q] = Ls[jj][tr + 16 * q];
-#pragma unroll
-      for (int p = 0; p < 8; ++p) x[p] = Xs[jj][tc * 8 + p];
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int p = 0; p < 8; ++p) acc[q][p] = fma(a[q], x[p], acc[q][p]);
+      for (int q = 0; q < kSB / 8; ++q)
+        if (q < nq) dmma_8x8x4(acc[q], a, Xs[(8 * q + g) * kXLd + s0 + t4]);
     }
     __syncthreads();
   }
+  const int i = r0 + 8 * warp + g;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int i = r0 + tr + 16 * q;
-    if (i >= m) continue;
+  for (int q = 0; q < kSB / 8; ++q)
 #pragma unroll
-    for (int p = 0; p < 8; ++p) {
-      const int cc = tc * 8 + p;
-      if (cc < bs) Wf[i + static_cast<std::int64_t>(b + cc) * m] = static_cast<F>(acc[q][p]);
+    for (int h = 0; h < 2; ++h) {
+      const int c = 8 * q + 2 * t4 + h;
+      if (i < m && c < bs) Wf[static_cast<std::int64_t>(c) * m + i] = static_cast<F>(acc[q][h]);
     }
-  }
 }
 
 namespace {
@@ -748,19 +902,24 @@ int solve_coop_max_ctas(int device) {
 }
 
 template <class F>
-void launch_sb_build(const int2* sbl, int nsb, const int4* tiles, int ntiles, const SnDev* sn, const F* panels,
-                     const signed char* piv, F* W, cudaStream_t s) {
-  if (nsb <= 0) return;
-  constexpr std::size_t smem = sizeof(double) * (kSB * (kSB - 1) / 2 + kSB * (kSB + 1) / 2 + kSB);
+void launch_sb_build(const SbLists& l, const SnDev* sn, const F* panels, const signed char* piv, F* W,
+                     cudaStream_t s) {
   static std::once_flag configured;
   std::call_once(configured, [&] {
-    cudaFuncSetAttribute(k_sb_inverse<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaFuncSetAttribute(k_sb_inverse<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kInvSmem));
+    cudaFuncSetAttribute(k_sb_apply<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kApplySmem));
   });
-  note_launches(1);
-  k_sb_inverse<F><<<nsb, 256, smem, s>>>(sbl, sn, panels, piv, W);
-  if (ntiles > 0) {
+  if (l.nwide > 0) {
     note_launches(1);
-    k_sb_apply<F><<<ntiles, 256, 0, s>>>(tiles, sn, panels, piv, W);
+    k_sb_inverse<F><<<l.nwide, 256, kInvSmem, s>>>(l.wide, sn, panels, piv, W);
+  }
+  if (l.ntiles > 0) {
+    note_launches(1);
+    k_sb_apply<F><<<l.ntiles, 256, kApplySmem, s>>>(l.tiles, sn, panels, piv, W);
+  }
+  if (l.nnarrow > 0) {
+    note_launches(1);
+    k_sb_narrow<F><<<l.nnarrow, 256, 0, s>>>(l.narrow, sn, panels, piv, W);
   }
 }
 
@@ -822,8 +981,7 @@ cudaError_t launch_bwd_tiny(const SolveTask* tasks, int ntasks, const SnDev* sn,
   template void launch_solve_diag_flat<F>(std::int64_t, const std::int64_t*, const std::int32_t*, const F*,          \
                                           const signed char*, const std::int32_t*, double*, std::int64_t, int,        \
                                           cudaStream_t);                                                               \
-  template void launch_sb_build<F>(const int2*, int, const int4*, int, const SnDev*, const F*, const signed char*,    \
-                                   F*, cudaStream_t);                                                                  \
+  template void launch_sb_build<F>(const SbLists&, const SnDev*, const F*, const signed char*, F*, cudaStream_t);                                                                  \
   template cudaError_t launch_fwd_level<F>(const SolveTask*, int, bool, const SnDev*, const std::int32_t*,           \
                                            const ContribEntry*, const F*, const std::int32_t*, double*, std::int64_t,  \
                                            double*, const SweepChunks&, double*, int*, int*, cudaStream_t);            \

@@ -26,10 +26,23 @@ void launch_solve_diag_flat(std::int64_t npiv, const std::int64_t* dpos, const s
 // Super-blocks of kSB pivots per front; their solve operator W (L_BB^{-1} on the diagonal block,
 // L L_BB^{-1} below it) is built once per factorization by launch_sb_build.
 constexpr int kSB = 128;
-// sbl: (front, super-block) pairs; tiles: (front, super-block, first row) of the 64-row tiles below
+// Super-blocks of at most kSbNarrow pivots are built by one kernel, in CTAs of kNarrowRows rows (narrow:
+// front, super-block, first row, 1 where the inverse is written too); a tensor tile of 64 x 128 leaves
+// them idle, and they are most of a tree's. The others take an inverse per (front, super-block) and a
+// tile per 64 rows below it (front, super-block, first row).
+constexpr int kSbNarrow = 32;
+constexpr int kNarrowRows = 256;
+struct SbLists {
+  const int2* wide;
+  int nwide;
+  const int4* tiles;
+  int ntiles;
+  const int4* narrow;
+  int nnarrow;
+};
 template <class F>
-void launch_sb_build(const int2* sbl, int nsb, const int4* tiles, int ntiles, const SnDev* sn, const F* panels,
-                     const signed char* piv, F* W, cudaStream_t s);
+void launch_sb_build(const SbLists& lists, const SnDev* sn, const F* panels, const signed char* piv, F* W,
+                     cudaStream_t s);
 // co-resident CTAs of the sweep kernels (the bound of a cooperative level launch)
 int solve_coop_max_ctas(int device);
 // One level of the forward / backward sweep: one CTA per task (front, rank, nr, work offset) and
