@@ -21,29 +21,115 @@ void cuda_check(cudaError_t e, const char* what);
 
 namespace {
 
-// One warp per row; each lane handles a stride of the row's entries, all p columns at once.
-template <int P>
-__global__ void k_spmm(std::int64_t n, const std::int64_t* rp, const std::int32_t* ci, const double* v, const double* x,
-                       std::int64_t ldx, double* y, std::int64_t ldy, int p, double alpha, double beta) {
-  const int lane = threadIdx.x & 31;
-  const std::int64_t warp = (blockIdx.x * static_cast<std::int64_t>(blockDim.x) + threadIdx.x) >> 5;
-  const std::int64_t nwarps = (static_cast<std::int64_t>(gridDim.x) * blockDim.x) >> 5;
-  for (std::int64_t i = warp; i < n; i += nwarps) {
-    double acc[P];
+// Rows of a CSR product are summed by four lanes each, eight rows a warp: the entries of a row are read
+// by neighbouring lanes, the gathers of neighbouring rows fall into the same lines, and the partial
+// sums take two shuffle steps. A curl-curl row has at most 13 entries: a warp per row left 19 lanes idle
+// and spent most of its time in five-step reductions (the residual of 8 columns at n = 21,660: 122 us,
+// now 11). Rows of more than kLongRow entries are summed by the whole warp.
+constexpr int kLongRow = 128;
+
+// f(value, column) for this lane's entries of row i (quad: every 4th; rows beyond kLongRow are left to
+// the warp). Four entries are read ahead of their gathers: a curl-curl row is one round of latencies.
+template <class Fn>
+__device__ __forceinline__ void quad_entries(const std::int64_t* rp, const std::int32_t* ci, const double* v,
+                                             std::int64_t i, bool in, Fn&& f) {
+  constexpr int kAhead = 4;
+  const int sub = threadIdx.x & 3;
+  const std::int64_t q0 = in ? rp[i] : 0, q1 = in ? rp[i + 1] : 0;
+  if (q1 - q0 > kLongRow) return;
+  for (std::int64_t q = q0 + sub; q < q1; q += 4 * kAhead) {
+    double a[kAhead];
+    std::int32_t j[kAhead];
 #pragma unroll
-    for (int r = 0; r < P; ++r) acc[r] = 0.0;
-    for (std::int64_t q = rp[i] + lane; q < rp[i + 1]; q += 32) {
-      const double a = v[q];
-      const std::int64_t j = ci[q];
-#pragma unroll
-      for (int r = 0; r < P; ++r)
-        if (r < p) acc[r] += a * x[j + r * ldx];
+    for (int u = 0; u < kAhead; ++u) {
+      a[u] = q + 4 * u < q1 ? v[q + 4 * u] : 0.0;
+      j[u] = q + 4 * u < q1 ? ci[q + 4 * u] : -1;
     }
 #pragma unroll
-    for (int r = 0; r < P; ++r) {
-      if (r >= p) break;
-      const double s = warp_sum(acc[r]);
-      if (lane == 0) y[i + r * ldy] = alpha * s + (beta == 0.0 ? 0.0 : beta * y[i + r * ldy]);
+    for (int u = 0; u < kAhead; ++u)
+      if (j[u] >= 0) f(a[u], j[u]);
+  }
+}
+
+// The quad's sums of P columns, scattered: lane sub keeps columns quad_col<P>() .. + P / 4 (P < 4: one
+// column, held by several lanes) in a[0 ..]; half the shuffles of a full reduction per step.
+template <int P>
+__device__ __forceinline__ void quad_scatter(double (&a)[P]) {
+  int width = P;
+#pragma unroll
+  for (int o = 2; o > 0; o >>= 1) {
+    const bool up = (threadIdx.x & o) != 0;
+    if (width > 1) {
+      width /= 2;
+#pragma unroll
+      for (int c = 0; c < P / 2; ++c)
+        if (c < width) {
+          const double send = up ? a[c] : a[c + width], keep = up ? a[c + width] : a[c];
+          a[c] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    } else {
+      a[0] += __shfl_xor_sync(0xffffffffu, a[0], o);
+    }
+  }
+}
+template <int P>
+__device__ __forceinline__ int quad_col() {
+  const int sub = threadIdx.x & 3;
+  return P >= 4 ? sub * (P / 4) : (P == 2 ? sub >> 1 : 0);
+}
+
+// the warp's long rows, one after another: f(row, owner) with the row's quad `owner`
+template <class Fn>
+__device__ __forceinline__ void long_rows(const std::int64_t* rp, std::int64_t row0, std::int64_t n, Fn&& f) {
+  const int lane = threadIdx.x & 31;
+  const std::int64_t i = row0 + (lane >> 2);
+  unsigned m = __ballot_sync(0xffffffffu, (lane & 3) == 0 && i < n && rp[i + 1] - rp[i] > kLongRow);
+  while (m) {
+    const int o = __ffs(m) - 1;
+    m &= m - 1;
+    f(row0 + (o >> 2), o >> 2);
+  }
+}
+
+template <int P>
+__global__ void __launch_bounds__(256, 3) k_spmm(std::int64_t n, const std::int64_t* rp, const std::int32_t* ci,
+                                                 const double* v, const double* x, std::int64_t ldx, double* y,
+                                                 std::int64_t ldy, int p, double alpha, double beta) {
+  constexpr int K = P >= 4 ? P / 4 : 1;
+  const int lane = threadIdx.x & 31, c0 = quad_col<P>();
+  const std::int64_t warp = (blockIdx.x * static_cast<std::int64_t>(blockDim.x) + threadIdx.x) >> 5;
+  const std::int64_t nwarps = (static_cast<std::int64_t>(gridDim.x) * blockDim.x) >> 5;
+  std::int64_t off[P];  // columns beyond p repeat column 0: read, never stored
+#pragma unroll
+  for (int c = 0; c < P; ++c) off[c] = c < p ? c * ldx : 0;
+  for (std::int64_t row0 = 8 * warp; row0 < n; row0 += 8 * nwarps) {
+    const std::int64_t i = row0 + (lane >> 2);
+    double acc[P];
+#pragma unroll
+    for (int c = 0; c < P; ++c) acc[c] = 0.0;
+    auto add = [&](double a, std::int64_t j, double (&t)[P]) {
+      const double* xj = x + j;
+#pragma unroll
+      for (int c = 0; c < P; ++c) t[c] = fma(a, xj[off[c]], t[c]);
+    };
+    quad_entries(rp, ci, v, i, i < n, [&](double a, std::int64_t j) { add(a, j, acc); });
+    long_rows(rp, row0, n, [&](std::int64_t row, int owner) {
+      double t[P];
+#pragma unroll
+      for (int c = 0; c < P; ++c) t[c] = 0.0;
+      for (std::int64_t q = rp[row] + lane; q < rp[row + 1]; q += 32) add(v[q], ci[q], t);
+#pragma unroll
+      for (int c = 0; c < P; ++c) {
+        const double w = warp_sum(t[c]);
+        if (lane == 4 * owner) acc[c] = w;
+      }
+    });
+    quad_scatter(acc);
+#pragma unroll
+    for (int u = 0; u < K; ++u) {
+      const int c = c0 + u;
+      if (c < p && i < n && (P >= 4 || (lane & (P == 2 ? 1 : 3)) == 0))
+        y[i + c * ldy] = alpha * acc[u] + (beta == 0.0 ? 0.0 : beta * y[i + c * ldy]);
     }
   }
 }
@@ -182,7 +268,7 @@ __global__ void k_fill_normal(std::int64_t n, int p, double* y, std::int64_t ldy
   }
 }
 
-// Shifted residual of a shift-invert solve, one warp per row and all P columns at once:
+// Shifted residual of a shift-invert solve, four lanes per row and all P columns at once:
 //   r(i, c) = (B w_c)(i) - (A y_c)(i),  w = x + sigma y  (B = null: B = I),
 //   s(i, c) = (|B| |w_c|)(i) + (|A| |y_c|)(i),
 // and the componentwise backward error omega_c = max_i |r(i, c)| / s(i, c) with 0/0 = 0, r/0 = inf and
@@ -190,72 +276,101 @@ __global__ void k_fill_normal(std::int64_t n, int p, double* y, std::int64_t ldy
 // include/hsolve/sparse.hpp:157-174). omega must hold zeros at launch; the maximum is taken by an
 // integer atomic max on the bit patterns of non-negative doubles (order independent).
 template <int P>
-__global__ void k_shifted_residual(std::int64_t n, const std::int64_t* arp, const std::int32_t* aci, const double* av,
-                                   const std::int64_t* brp, const std::int32_t* bci, const double* bv, double sigma,
-                                   const double* x, std::int64_t ldx, const double* y, std::int64_t ldy, double* r,
-                                   std::int64_t ldr, int p, unsigned long long* omega) {
-  const int lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(256, 3) k_shifted_residual(std::int64_t n, const std::int64_t* arp,
+                                                             const std::int32_t* aci, const double* av,
+                                                             const std::int64_t* brp, const std::int32_t* bci,
+                                                             const double* bv, double sigma, const double* x,
+                                                             std::int64_t ldx, const double* y, std::int64_t ldy,
+                                                             double* r, std::int64_t ldr, int p,
+                                                             unsigned long long* omega) {
+  constexpr int K = P >= 4 ? P / 4 : 1;
+  const int lane = threadIdx.x & 31, c0 = quad_col<P>();
   const std::int64_t warp = (blockIdx.x * static_cast<std::int64_t>(blockDim.x) + threadIdx.x) >> 5;
   const std::int64_t nwarps = (static_cast<std::int64_t>(gridDim.x) * blockDim.x) >> 5;
-  double om[P];
+  const auto xoff = [&](int c) { return c < p ? c * ldx : 0; };  // columns beyond p repeat column 0
+  std::int64_t yoff[P];
 #pragma unroll
-  for (int c = 0; c < P; ++c) om[c] = 0.0;
-  for (std::int64_t i = warp; i < n; i += nwarps) {
+  for (int c = 0; c < P; ++c) yoff[c] = c < p ? c * ldy : 0;
+  double om[K];
+#pragma unroll
+  for (int u = 0; u < K; ++u) om[u] = 0.0;
+  for (std::int64_t row0 = 8 * warp; row0 < n; row0 += 8 * nwarps) {
+    const std::int64_t i = row0 + (lane >> 2);
+    const bool in = i < n;
     double ra[P], sa[P];
 #pragma unroll
     for (int c = 0; c < P; ++c) { ra[c] = 0.0; sa[c] = 0.0; }
-    for (std::int64_t q = arp[i] + lane; q < arp[i + 1]; q += 32) {
-      const double a = av[q];
-      const std::int64_t j = aci[q];
+    auto add_a = [&](double a, std::int64_t j, double (&rr)[P], double (&ss)[P]) {
+      const double* yj = y + j;
 #pragma unroll
-      for (int c = 0; c < P; ++c)
-        if (c < p) {
-          const double yj = y[j + c * ldy];
-          ra[c] = fma(-a, yj, ra[c]);
-          sa[c] = fma(fabs(a), fabs(yj), sa[c]);
-        }
-    }
-    if (brp) {
-      for (std::int64_t q = brp[i] + lane; q < brp[i + 1]; q += 32) {
-        const double b = bv[q];
-        const std::int64_t j = bci[q];
-#pragma unroll
-        for (int c = 0; c < P; ++c)
-          if (c < p) {
-            const double wj = fma(sigma, y[j + c * ldy], x[j + c * ldx]);
-            ra[c] = fma(b, wj, ra[c]);
-            sa[c] = fma(fabs(b), fabs(wj), sa[c]);
-          }
+      for (int c = 0; c < P; ++c) {
+        const double t = yj[yoff[c]];
+        rr[c] = fma(-a, t, rr[c]);
+        ss[c] = fma(fabs(a), fabs(t), ss[c]);
       }
-    } else if (lane == 0) {
+    };
+    auto add_b = [&](double b, std::int64_t j, double (&rr)[P], double (&ss)[P]) {
 #pragma unroll
-      for (int c = 0; c < P; ++c)
-        if (c < p) {
-          const double wi = fma(sigma, y[i + c * ldy], x[i + c * ldx]);
-          ra[c] += wi;
-          sa[c] += fabs(wi);
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < P; ++c) {
-      if (c >= p) break;
-      const double rs = warp_sum(ra[c]);
-      const double ss = warp_sum(sa[c]);
-      if (lane == 0) {
-        if (r) r[i + c * ldr] = rs;
-        const double ar = fabs(rs);
-        double w;
-        if (!isfinite(rs) || !isfinite(ss)) w = CUDART_INF;
-        else if (ss > 0.0) w = ar / ss;
-        else w = ar > 0.0 ? CUDART_INF : 0.0;
-        om[c] = fmax(om[c], w);
+      for (int c = 0; c < P; ++c) {
+        const double w = fma(sigma, y[j + yoff[c]], x[j + xoff(c)]);
+        rr[c] = fma(b, w, rr[c]);
+        ss[c] = fma(fabs(b), fabs(w), ss[c]);
       }
+    };
+    quad_entries(arp, aci, av, i, in, [&](double a, std::int64_t j) { add_a(a, j, ra, sa); });
+    if (brp) quad_entries(brp, bci, bv, i, in, [&](double b, std::int64_t j) { add_b(b, j, ra, sa); });
+    auto by_warp = [&](const std::int64_t* rp, const std::int32_t* ci, const double* v, auto&& add) {
+      long_rows(rp, row0, n, [&](std::int64_t row, int owner) {
+        double rr[P], ss[P];
+#pragma unroll
+        for (int c = 0; c < P; ++c) { rr[c] = 0.0; ss[c] = 0.0; }
+        for (std::int64_t q = rp[row] + lane; q < rp[row + 1]; q += 32) add(v[q], ci[q], rr, ss);
+#pragma unroll
+        for (int c = 0; c < P; ++c) {
+          const double tr = warp_sum(rr[c]), ts = warp_sum(ss[c]);
+          if (lane == 4 * owner) { ra[c] += tr; sa[c] += ts; }
+        }
+      });
+    };
+    by_warp(arp, aci, av, add_a);
+    if (brp) by_warp(brp, bci, bv, add_b);
+    quad_scatter(ra);
+    quad_scatter(sa);
+#pragma unroll
+    for (int u = 0; u < K; ++u) {
+      const int c = c0 + u;
+      if (c >= p || !in) continue;
+      double rs = ra[u], ss = sa[u];
+      if (!brp) {
+        const double w = fma(sigma, y[i + c * ldy], x[i + c * ldx]);
+        rs += w;
+        ss += fabs(w);
+      }
+      if (r && (P >= 4 || (lane & (P == 2 ? 1 : 3)) == 0)) r[i + c * ldr] = rs;
+      const double ar = fabs(rs);
+      double w;
+      if (!isfinite(rs) || !isfinite(ss)) w = CUDART_INF;
+      else if (ss > 0.0) w = ar / ss;
+      else w = ar > 0.0 ? CUDART_INF : 0.0;
+      om[u] = fmax(om[u], w);
     }
   }
-  if (omega && lane == 0) {
+  if (omega) {
+    // one atomic per column and CTA
+    __shared__ double part[8][P];
 #pragma unroll
-    for (int c = 0; c < P; ++c)
-      if (c < p && om[c] > 0.0) atomic_max_nonneg(&omega[c], om[c]);
+    for (int u = 0; u < K; ++u) {
+      double w = om[u];
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) w = fmax(w, __shfl_xor_sync(0xffffffffu, w, o));
+      if (lane < 4) part[threadIdx.x >> 5][c0 + u] = w;
+    }
+    __syncthreads();
+    if (threadIdx.x < P && static_cast<int>(threadIdx.x) < p) {
+      double w = 0.0;
+      for (int q = 0; q < 8; ++q) w = fmax(w, part[q][threadIdx.x]);
+      if (w > 0.0) atomic_max_nonneg(&omega[threadIdx.x], w);
+    }
   }
 }
 
@@ -281,11 +396,6 @@ __global__ void k_copy_cols_masked(std::int64_t n, int p, unsigned mask, const d
   }
 }
 
-// bits of a non-negative double array (atomic max slots) -> doubles, in place
-__global__ void k_bits_to_double(int p, unsigned long long* w) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < p) reinterpret_cast<double*>(w)[c] = __longlong_as_double(static_cast<long long>(w[c]));
-}
 
 // r = a - lam .* b (column c uses lam[c]); y holds r
 __global__ void k_residual_cols(std::int64_t n, int p, const double* ax, std::int64_t lda, const double* bx,
@@ -336,7 +446,7 @@ void spmm(const CsrDev& M, const double* x, std::int64_t ldx, double* y, std::in
           double beta, cudaStream_t s) {
   if (p <= 0 || M.n == 0) return;
   const int threads = 256;
-  const int blocks = grid_for(M.n * 32, threads);
+  const int blocks = grid_for(M.n * 4, threads);
   for (int c0 = 0; c0 < p; c0 += 8) {
     const int pc = p - c0 < 8 ? p - c0 : 8;
     const double* xc = x + c0 * ldx;
@@ -465,7 +575,7 @@ void shifted_residual(const CsrDev& A, const CsrDev* B, double sigma, const doub
                       cudaStream_t s) {
   if (p <= 0 || A.n == 0) return;
   const int threads = 256;
-  const int blocks = grid_for(A.n * 32, threads);
+  const int blocks = grid_for(A.n * 4, threads);
   if (omega) cuda_check(cudaMemsetAsync(omega, 0, static_cast<std::size_t>(p) * sizeof(double), s), "memset omega");
   for (int c0 = 0; c0 < p; c0 += 8) {
     const int pc = p - c0 < 8 ? p - c0 : 8;
@@ -485,10 +595,6 @@ void shifted_residual(const CsrDev& A, const CsrDev* B, double sigma, const doub
       k_shifted_residual<4><<<blocks, threads, 0, s>>>(A.n, A.rp, A.ci, A.v, brp, bci, bvv, sigma, xc, ldx, yc, ldy, rc, ldr, pc, oc);
     else
       k_shifted_residual<8><<<blocks, threads, 0, s>>>(A.n, A.rp, A.ci, A.v, brp, bci, bvv, sigma, xc, ldx, yc, ldy, rc, ldr, pc, oc);
-  }
-  if (omega) {
-    note_launches(1);
-    k_bits_to_double<<<(p + 127) / 128, 128, 0, s>>>(p, reinterpret_cast<unsigned long long*>(omega));
   }
 }
 
