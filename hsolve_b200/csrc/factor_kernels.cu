@@ -960,6 +960,33 @@ __device__ void app_init(AppFront<R>& F, int rank, int nr) {
   }
 }
 
+// Rank 0: the factored block at column p (order w, in Bs) to the front and to the panel's arrays.
+template <class R>
+__device__ void app_publish_block(AppFront<R>& F, int p, int w, const R* Bs, const int* slab, const signed char* spv,
+                                  const StepShared& bst) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (__syncthreads_or(threadIdx.x < w && slab[threadIdx.x] != static_cast<int>(threadIdx.x))) {
+    // the block's rows were swapped: its pivot labels follow
+    int old = 0;
+    if (threadIdx.x < w) old = F.plab[p + slab[threadIdx.x]];
+    __syncthreads();
+    if (threadIdx.x < w) F.plab[p + threadIdx.x] = old;
+  }
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    const int c2 = warp + 8 * s;
+    if (lane >= c2 && lane < w) F.f.at(p + lane, p + c2) = Bs[lane + c2 * kNB];
+    F.B[lane + c2 * kNB] = Bs[lane + c2 * kNB];
+  }
+  for (int t = threadIdx.x; t < kNB; t += blockDim.x) {
+    F.lab[t] = slab[t];
+    F.pv[t] = spv[t];
+    F.cmax[t] = 0ull;
+    F.rmax[t] = 0ull;
+  }
+  if (threadIdx.x == 0) F.ctrl->eb = bst.j;
+}
+
 // Rank 0: decide what the next panel is (stop = 1: front finished), and factorize its diagonal block
 // with block-restricted threshold Bunch-Kaufman; permute the L rows of the block; publish to scratch.
 template <class R>
@@ -1042,7 +1069,6 @@ __device__ void app_control_and_block(AppFront<R>& F, const FactorParams& prm, d
     if (r > p + 1) front_swap(F.f, p + 1, r, F.plab);
     __syncthreads();
   }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   RegTri<kNB, kAppThreads, R> y;
   y.place();
 #pragma unroll
@@ -1053,27 +1079,7 @@ __device__ void app_control_and_block(AppFront<R>& F, const FactorParams& prm, d
   if (threadIdx.x == 0) bk_begin(bst, w);
   __syncthreads();
   block_bk(y, Bs, qs, w, force, prm.u, thr, slab, spv, bst);
-  const int eb = bst.j;
-  if (__syncthreads_or(threadIdx.x < w && slab[threadIdx.x] != static_cast<int>(threadIdx.x))) {
-    // the block's rows were swapped: its pivot labels follow
-    int old = 0;
-    if (threadIdx.x < w) old = F.plab[p + slab[threadIdx.x]];
-    __syncthreads();
-    if (threadIdx.x < w) F.plab[p + threadIdx.x] = old;
-  }
-#pragma unroll
-  for (int s = 0; s < 4; ++s) {
-    const int c2 = warp + 8 * s;
-    if (lane >= c2 && lane < w) F.f.at(p + lane, p + c2) = Bs[lane + c2 * kNB];
-    F.B[lane + c2 * kNB] = Bs[lane + c2 * kNB];
-  }
-  for (int t = threadIdx.x; t < kNB; t += blockDim.x) {
-    F.lab[t] = slab[t];
-    F.pv[t] = spv[t];
-    F.cmax[t] = 0ull;
-    F.rmax[t] = 0ull;
-  }
-  if (threadIdx.x == 0) c->eb = eb;
+  app_publish_block(F, p, w, Bs, slab, spv, bst);
 }
 
 // All ranks: rows [p+w, m) solved against the block (L21 = F21 P L11^-T D^-1), backup, column maxima.
@@ -1389,9 +1395,10 @@ __device__ __forceinline__ bool app_flushes(int p, int w, int q, int lim, int fb
 // the same output ownership per thread, and accumulate with FP32 FMAs (there is no FP32 tensor
 // instruction with full FP32 operands; the FP64 refinement of every solve absorbs FP32 rounding).
 //
-// With look-ahead (la: the panel was accepted whole and the next one follows directly), rank 0 takes
-// only tile 0, which holds the next panel's diagonal block, so that it can factorize that block
-// while the other ranks finish the remaining tiles.
+// With look-ahead (la: the panel was accepted whole and the next one follows directly), rank 0 updates
+// and factorizes the next panel's diagonal block first (app_next_block): that block is left out here, and
+// rank 0 takes the last tiles of the list, fewer than the others by what its block costs (about 8 us: two
+// tiles of 128 pivots, five of 32).
 struct UpdTile {
   int tile, i0, j0;
 };
@@ -1414,11 +1421,16 @@ __device__ void app_update(AppFront<R>& F, const StepView& v, int rank, int nr, 
   const int rbase = (warp & 3) * 16, cbase = (warp >> 2) * 32;
   const int Kpad = (K + 3) & ~3;
   const int nk = (K + kUpdChunk - 1) / kUpdChunk;
-  // tiles of this rank: round-robin, or with look-ahead tile 0 for rank 0 and the rest over ranks 1..
+  // tiles [tfirst, tend) of this rank by tstep: round-robin, or with look-ahead the last t0 for rank 0
+  // and the others over ranks 1..
   const bool split = la && nr > 1;
-  const int tfirst = split ? (rank == 0 ? 0 : rank) : rank;
-  const int tstep = split ? (rank == 0 ? ntiles : nr - 1) : nr;
-  if (tfirst >= ntiles) return;
+  const int behind = K > 64 ? 2 : (K > 32 ? 3 : 5);
+  const int t0 = split ? max(0, (ntiles + behind) / nr - behind) : 0;
+  const int tfirst = split ? (rank == 0 ? ntiles - t0 : rank - 1) : rank;
+  const int tend = split && rank > 0 ? ntiles - t0 : ntiles;
+  const int tstep = split ? (rank == 0 ? 1 : nr - 1) : nr;
+  if (tfirst >= tend) return;
+  const int skip = la ? min(kNB, lim - from) + from : from;  // rows (and columns) below: the next block
   auto locate = [&](UpdTile& t) {
     int ti, tj;
     if (nct == nt) {
@@ -1459,13 +1471,13 @@ __device__ void app_update(AppFront<R>& F, const StepView& v, int rank, int nr, 
   ct = ft;
   int fk = 0, fst = 0, cst = 0;
   auto fetch_next = [&]() {
-    if (ft.tile < ntiles) {
+    if (ft.tile < tend) {
       issue(ft, fk, fst);
       fst = fst + 1 == kUpdStages ? 0 : fst + 1;
       if (++fk == nk) {
         fk = 0;
         ft.tile += tstep;
-        if (ft.tile < ntiles) locate(ft);
+        if (ft.tile < tend) locate(ft);
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -1473,11 +1485,11 @@ __device__ void app_update(AppFront<R>& F, const StepView& v, int rank, int nr, 
   __syncthreads();  // the staging area's last users are done
 #pragma unroll
   for (int u = 0; u < kUpdStages - 1; ++u) fetch_next();
-  while (ct.tile < ntiles) {
+  while (ct.tile < tend) {
     const int i0 = ct.i0, j0 = ct.j0;
     // warps whose 32 columns all lie at or beyond col_hi (the second half of a panel's tile) or
-    // whose 16 rows all lie above their first column have nothing to update
-    const bool idle = j0 + cbase >= col_hi || i0 + rbase + 15 < j0 + cbase;
+    // whose 16 rows all lie above their first column or in the next block have nothing to update
+    const bool idle = j0 + cbase >= col_hi || i0 + rbase + 15 < max(j0 + cbase, skip);
     // this thread's C entries (rows rbase + 8a + g, columns cbase + 8b + 2 t4 + e)
     R* colp[4][2];
     R cv[2][4][2], acc[2][4][2];
@@ -1490,7 +1502,7 @@ __device__ void app_update(AppFront<R>& F, const StepView& v, int rank, int nr, 
 #pragma unroll
         for (int a = 0; a < 2; ++a) {
           const int i = i0 + rbase + 8 * a + g;
-          cv[a][b][e] = (colp[b][e] && i < m && cc <= i) ? colp[b][e][i] : R(0);
+          cv[a][b][e] = (colp[b][e] && i < m && cc <= i && i >= skip) ? colp[b][e][i] : R(0);
           acc[a][b][e] = R(0);
         }
       }
@@ -1543,11 +1555,11 @@ __device__ void app_update(AppFront<R>& F, const StepView& v, int rank, int nr, 
 #pragma unroll
         for (int a = 0; a < 2; ++a) {
           const int i = i0 + rbase + 8 * a + g;
-          if (colp[b][e] && i < m && cc <= i) colp[b][e][i] = cv[a][b][e] - acc[a][b][e];
+          if (colp[b][e] && i < m && cc <= i && i >= skip) colp[b][e][i] = cv[a][b][e] - acc[a][b][e];
         }
       }
     ct.tile += tstep;
-    if (ct.tile < ntiles) locate(ct);
+    if (ct.tile < tend) locate(ct);
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
@@ -1586,6 +1598,76 @@ struct AppSmem {
   StepShared bst;
   int stop, q, ok;
 };
+
+// Rank 0, look-ahead: the panel at v was accepted whole and the next one follows directly. Applies the
+// pending pivots to the next panel's diagonal block in the registers that its factorization works in (the
+// accumulator layout of the tensor instruction), factorizes it and publishes the next step. Done before the
+// rank's share of the update: the block is on the panel chain, the update is not. (As the first 64 x 64
+// tile of the update, written back and read again, it took 5.8 us of a root panel, and the control block's
+// global reads and the swap logic 2 more.)
+template <class R>
+__device__ void app_next_block(AppFront<R>& F, const StepView& v, int slot, const FactorParams& prm, double thr,
+                               AppSmem<R>& sm, R* stage) {
+  constexpr int kLd = kNB + 4;  // 4 (mod 16): conflict-free fragment reads
+  const int m = F.f.m, fb = v.fb, p = v.p + v.w, w = min(kNB, v.lim - p), K = p - fb;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
+  const int Kpad = (K + 7) & ~7;
+  set_slot(F, slot);
+  R* Ls = stage;
+  R* Ws = stage + kKB * kLd;
+  __syncthreads();  // the staging area's last users are done
+  for (int s = warp; s < Kpad; s += kAppThreads / 32) {
+    const bool in = s < K && lane < w;
+    const std::int64_t at = static_cast<std::int64_t>(in ? s : 0) * m + (in ? p + lane : p);
+    cp_async_elem(&Ls[s * kLd + lane], F.f.panel + static_cast<std::int64_t>(fb) * m + at, in);
+    cp_async_elem(&Ws[s * kLd + lane], F.wd + at, in);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  RegTri<kNB, kAppThreads, R> y;
+  y.place();
+#pragma unroll
+  for (int s = 0; s < y.PER; ++s) y.v[s][0] = y.v[s][1] = R(0);
+  y.each([&](R& x, int i, int c) { if (i < w) x = F.f.at(p + i, p + c); });
+  for (int t = threadIdx.x; t < w; t += blockDim.x) sm.slab[t] = t;
+  if (threadIdx.x == 0) {
+    AppCtrl* c = F.ctrl;
+    c->p = p;
+    c->w = w;
+    c->prog = 1;
+    c->force = 0;
+    c->stop = 0;
+    if (app_flushes(v.p, v.w, v.w, v.lim, fb)) c->fb = p;
+    bk_begin(sm.bst, w);
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+#pragma unroll
+  for (int s = 0; s < y.PER; ++s) {
+    if (y.c0[s] == y.kNone) continue;
+    const int rb = y.r0[s] - g, cb = y.c0[s] - 2 * t4;
+    R acc[2][2] = {};  // even and odd groups of four pivots: two chains
+    if constexpr (sizeof(R) == 8) {
+      for (int s0 = 0; s0 < Kpad; s0 += 8)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int k = (s0 + 4 * h + t4) * kLd;
+          dmma_m8n8k4(acc[h][0], acc[h][1], Ls[k + rb + g], Ws[k + cb + g]);
+        }
+    } else {
+      for (int k = 0; k < K; ++k) {
+        const R l = Ls[k * kLd + y.r0[s]];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) acc[0][e] = fma(l, Ws[k * kLd + y.c0[s] + e], acc[0][e]);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) y.v[s][e] -= acc[0][e] + acc[1][e];
+  }
+  y.each([&](R& x, int i, int c) { if (i < w) F.Borig[i + c * kNB] = x; });
+  __syncthreads();
+  block_bk(y, sm.Bs, sm.qs, w, false, prm.u, thr, sm.slab, sm.spv, sm.bst);
+  app_publish_block(F, p, w, sm.Bs, sm.slab, sm.spv, sm.bst);
+}
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
@@ -1633,7 +1715,7 @@ __device__ bool front_barrier(int* bar, int nr, unsigned long long* timeouts, in
 //   [control: rank 0 advances past the previous panel and factorizes the next block] barrier
 //   rows (all) barrier  accept (all, identical)  [restore (all) barrier]  update (all) barrier
 // and when a panel is accepted whole and the next one follows directly (look-ahead), rank 0
-// advances and factorizes the next block right after its update tile, so that the control phase
+// advances and factorizes the next block before its share of the update, so that the control phase
 // and its barrier are skipped. Alternate panels use alternate per-panel arrays, so the next
 // block's arrays never overlap the ones slower CTAs still read.
 template <bool kCoop, class R>
@@ -1670,14 +1752,8 @@ __device__ void app_front(AppFront<R>& F, int rank, int nr, const FactorParams& 
       if (!sync()) break;
     }
     la = q == v.w && v.p + v.w < v.lim;
+    if (la && rank == 0) app_next_block(F, v, (j + 1) & 1, prm, thr, sm, stage);
     app_update(F, v, rank, nr, q, la, stage);
-    if (la && rank == 0) {
-      __syncthreads();
-      app_advance(F, q);
-      set_slot(F, (j + 1) & 1);
-      app_control_and_block(F, prm, thr, sm.Bs, sm.qs, sm.slab, sm.spv, sm.bst, &sm.stop, cnt, failed,
-                            level_done);
-    }
     if (!sync()) break;
     qprev = q;
     ++j;
