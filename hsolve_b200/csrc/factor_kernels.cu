@@ -53,6 +53,13 @@ __device__ __forceinline__ void cp_async_elem(R* dst, const R* src, bool valid) 
   }
 }
 
+// the same to a shared-memory address, of `size` bytes (sizeof(R), or 0: filled with zero)
+template <class R>
+__device__ __forceinline__ void cp_async_sized(unsigned dst, const R* src, int size) {
+  if constexpr (sizeof(R) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(size) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(size) : "memory");
+}
+
 // ------------------------------------------------------------------ scaling and assembly
 
 __global__ void k_fill(double* x, std::int64_t n, double v) {
@@ -1400,7 +1407,7 @@ __device__ __forceinline__ bool app_flushes(int p, int w, int q, int lim, int fb
 // rank 0 takes the last tiles of the list, fewer than the others by what its block costs (about 8 us: two
 // tiles of 128 pivots, five of 32).
 struct UpdTile {
-  int tile, i0, j0;
+  int tile, ti, tj;
 };
 
 template <class R>
@@ -1431,53 +1438,60 @@ __device__ void app_update(AppFront<R>& F, const StepView& v, int rank, int nr, 
   const int tstep = split ? (rank == 0 ? 1 : nr - 1) : nr;
   if (tfirst >= tend) return;
   const int skip = la ? min(kNB, lim - from) + from : from;  // rows (and columns) below: the next block
-  auto locate = [&](UpdTile& t) {
-    int ti, tj;
-    if (nct == nt) {
-      ti = static_cast<int>((sqrtf(8.0f * static_cast<float>(t.tile) + 1.0f) - 1.0f) * 0.5f);
-      while ((ti + 1) * (ti + 2) / 2 <= t.tile) ++ti;
-      while (ti * (ti + 1) / 2 > t.tile) --ti;
-      tj = t.tile - ti * (ti + 1) / 2;
-    } else {
-      int rest = t.tile;
-      tj = 0;
-      while (rest >= nt - tj) { rest -= nt - tj; ++tj; }
-      ti = tj + rest;
+  // the tile `step` further on, column by column: (ti, tj) with tj <= ti < nt
+  auto forward = [&](UpdTile& t, int step) {
+    t.tile += step;
+    t.ti += step;
+    while (t.ti >= nt && t.tj < nct) {
+      ++t.tj;
+      t.ti += t.tj - nt;
     }
-    t.i0 = from + ti * kTile;
-    t.j0 = from + tj * kTile;
   };
-  // chunk `kc` of tile `t` into stage `st`: a thread copies tile row r, pivots sg, sg + 4, ...
-  const R* lpan = F.f.panel + static_cast<std::int64_t>(fb) * m;
+  // a thread copies tile row r, pivots sg, sg + 4, ... of a chunk: pointers that advance by four columns,
+  // the validity of the row in the copies' sizes
   const int r = threadIdx.x & (kTile - 1), sg = threadIdx.x >> 6;
-  auto issue = [&](const UpdTile& t, int kc, int st) {
-    R* Ls = stage + st * (2 * kUpdChunk * kUpdLd);
-    R* Ws = Ls + kUpdChunk * kUpdLd;
-    const int i = t.i0 + r, c = t.j0 + r;
-    const int li = i < m ? i : from, lc = c < col_hi ? c : from;
-    const int smin = c < rej_hi ? p - fb : 0;
-#pragma unroll
-    for (int u = 0; u < kUpdChunk / 4; ++u) {
-      const int sl = sg + 4 * u, s = kc * kUpdChunk + sl;
-      if (s >= Kpad) break;
-      const bool in = s < K;
-      const std::int64_t col = static_cast<std::int64_t>(in ? s : 0) * m;
-      cp_async_elem(&Ls[sl * kUpdLd + r], lpan + col + li, in && i < m);
-      cp_async_elem(&Ws[sl * kUpdLd + r], F.wd + col + lc, in && c < col_hi && s >= smin);
+  const std::int64_t step4 = 4 * static_cast<std::int64_t>(m);
+  const R* lsrc = nullptr;
+  const R* wsrc = nullptr;
+  int lsize = 0, wsize = 0, smin = 0;
+  auto aim = [&](const UpdTile& t) {
+    const int i = from + t.ti * kTile + r, c = from + t.tj * kTile + r;
+    lsize = i < m ? static_cast<int>(sizeof(R)) : 0;
+    wsize = c < col_hi ? static_cast<int>(sizeof(R)) : 0;
+    smin = c < rej_hi ? p - fb : 0;
+    lsrc = F.f.panel + static_cast<std::int64_t>(fb + sg) * m + (i < m ? i : from);
+    wsrc = F.wd + static_cast<std::int64_t>(sg) * m + (c < col_hi ? c : from);
+  };
+  const unsigned stage0 = static_cast<unsigned>(__cvta_generic_to_shared(stage)) +
+                          static_cast<unsigned>((sg * kUpdLd + r) * sizeof(R));
+  constexpr unsigned kStageBytes = 2 * kUpdChunk * kUpdLd * sizeof(R), kHalf = kUpdChunk * kUpdLd * sizeof(R);
+  auto issue = [&](int kc, int st) {
+    unsigned dst = stage0 + st * kStageBytes;
+    int s = kc * kUpdChunk + sg;
+    const int send = min(Kpad, (kc + 1) * kUpdChunk);
+#pragma unroll 8
+    for (; s < send; s += 4) {
+      const bool in = s < K;  // (a copy of no bytes reads nothing: the pointer is not followed)
+      cp_async_sized<R>(dst, lsrc, in ? lsize : 0);
+      cp_async_sized<R>(dst + kHalf, wsrc, in && s >= smin ? wsize : 0);
+      dst += 4 * kUpdLd * sizeof(R);
+      lsrc += step4;
+      wsrc += step4;
     }
   };
-  UpdTile ft{tfirst, 0, 0}, ct;  // the tile being fetched, and the one computed
-  locate(ft);
+  UpdTile ft{0, 0, 0}, ct;  // the tile being fetched, and the one computed
+  forward(ft, tfirst);
+  aim(ft);
   ct = ft;
   int fk = 0, fst = 0, cst = 0;
   auto fetch_next = [&]() {
     if (ft.tile < tend) {
-      issue(ft, fk, fst);
+      issue(fk, fst);
       fst = fst + 1 == kUpdStages ? 0 : fst + 1;
       if (++fk == nk) {
         fk = 0;
-        ft.tile += tstep;
-        if (ft.tile < tend) locate(ft);
+        forward(ft, tstep);
+        if (ft.tile < tend) aim(ft);
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -1486,7 +1500,7 @@ __device__ void app_update(AppFront<R>& F, const StepView& v, int rank, int nr, 
 #pragma unroll
   for (int u = 0; u < kUpdStages - 1; ++u) fetch_next();
   while (ct.tile < tend) {
-    const int i0 = ct.i0, j0 = ct.j0;
+    const int i0 = from + ct.ti * kTile, j0 = from + ct.tj * kTile;
     // warps whose 32 columns all lie at or beyond col_hi (the second half of a panel's tile) or
     // whose 16 rows all lie above their first column or in the next block have nothing to update
     const bool idle = j0 + cbase >= col_hi || i0 + rbase + 15 < max(j0 + cbase, skip);
@@ -1558,8 +1572,7 @@ __device__ void app_update(AppFront<R>& F, const StepView& v, int rank, int nr, 
           if (colp[b][e] && i < m && cc <= i && i >= skip) colp[b][e][i] = cv[a][b][e] - acc[a][b][e];
         }
       }
-    ct.tile += tstep;
-    if (ct.tile < tend) locate(ct);
+    forward(ct, tstep);
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
