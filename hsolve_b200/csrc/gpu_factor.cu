@@ -541,10 +541,12 @@ std::shared_ptr<FrontPlan> GpuFactor::make_plan() {
           std::vector<int> nr(app.size());
           int total = 0;
           for (std::size_t q = 0; q < app.size(); ++q) {
-            // about 16 tiles of 64 x 64 per CTA at the first panel: fewer CTAs wait at the front's
-            // barriers, which leaves SMs to concurrent requests (served throughput +11 % on the
-            // n = 1e5 box against 8 tiles, one request 2 % slower)
-            const double want = std::ceil(wts[q] / (2.0 * 64 * 64 * 16));
+            // about 2 tiles of 64 x 64 per CTA at the first panel: a front that has the device to
+            // itself (the top levels) is faster the more CTAs share its update (n = 21,660: 4.65 ms
+            // a factorization with 16 tiles, 3.65 with 8, 3.08 with 2 or 3; n = 109,744: 13.2, 12.5,
+            // 12.4; n = 291,359, whose top levels have more tiles than CTAs: unchanged). Shifts that
+            // are factorized at once get the shared budget's plan.
+            const double want = std::ceil(wts[q] / (2.0 * 64 * 64 * 2));
             nr[q] = static_cast<int>(std::max(1.0, std::min<double>(want, budget)));
             total += nr[q];
           }
