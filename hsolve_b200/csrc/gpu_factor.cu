@@ -36,9 +36,11 @@ struct AnalysisEntry {
 };
 
 constexpr std::size_t kAnalysisCacheEntries = 8;
-// panel entries per CTA of a solve sweep (fewer, busier CTAs: their waits hold fewer SMs from
-// concurrent requests)
-constexpr double kSolveEntriesPerCta = 32768.0;
+// Panel entries per CTA of a solve sweep. The sweeps are chains of latencies, and a chain is shorter the
+// more CTAs share a front's rows, but waiting CTAs hold SMs from concurrent requests: one column at
+// n = 10,064 takes 398 us with 32,768 entries a CTA, 298 with 8,192, 274 with 2,048; the served stream of six
+// workers makes 17.5, 17.0 and 14.8 solves/s.
+constexpr double kSolveEntriesPerCta = 8192.0;
 // most parts a backward chunk's contribution-row tiles are cut into (owner + helpers)
 constexpr int kSolveParts = 4;
 std::mutex g_analysis_mu;
@@ -481,7 +483,7 @@ std::shared_ptr<FrontPlan> GpuFactor::make_plan() {
         }
         // backward helpers: where the level's CTAs fit the co-resident bound with room to spare, the
         // contribution-row tiles of each chunk of the widest fronts are cut into up to kSolveParts
-        // parts (about 16 tiles per CTA), parts 1.. on helper CTAs
+        // parts (about 8 tiles per CTA, one per warp), parts 1.. on helper CTAs
         std::vector<int> parts(all.size(), 1);
         int used = 0;
         for (int v : nr) used += v;
@@ -496,7 +498,7 @@ std::shared_ptr<FrontPlan> GpuFactor::make_plan() {
             const SnDev& dd = sn[all[q]];
             const int nch = (dd.k + 31) / 32, t2 = (dd.m - dd.k + 31) / 32;
             if (nch == 0 || spare < nch) continue;
-            int want = std::min({kSolveParts, std::max(1, (t2 + 4 + 15) / 16), std::max(1, t2)});
+            int want = std::min({kSolveParts, std::max(1, (t2 + 4 + 7) / 8), std::max(1, t2)});
             want = std::min(want, 1 + spare / nch);
             parts[q] = want;
             spare -= nch * (want - 1);
