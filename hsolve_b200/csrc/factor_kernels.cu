@@ -74,9 +74,12 @@ __global__ void k_zero_u64(unsigned long long* x, std::int64_t n) {
     x[i] = 0ull;
 }
 
+// The kernels that form K = alpha A + beta B read (alpha, beta) = ab[0..1] from device memory, so that a
+// captured factorization serves every shift.
 // r[i] = max_j |d_i K_ij d_j| over both triangles (atomic max on non-negative doubles)
 __global__ void k_scale_rowmax(std::int64_t nnz, const std::int32_t* row, const std::int32_t* col, const double* a,
-                               const double* b, double alpha, double beta, const double* d, unsigned long long* r) {
+                               const double* b, const double* ab, const double* d, unsigned long long* r) {
+  const double alpha = ab[0], beta = ab[1];
   for (std::int64_t p = blockIdx.x * static_cast<std::int64_t>(blockDim.x) + threadIdx.x; p < nnz;
        p += static_cast<std::int64_t>(gridDim.x) * blockDim.x) {
     const std::int32_t i = row[p], j = col[p];
@@ -99,8 +102,9 @@ __global__ void k_scale_update(std::int64_t n, double* d, unsigned long long* r)
 // for the null-pivot threshold
 template <class R>
 __global__ void k_scatter(std::int64_t nnz, const std::int32_t* row, const std::int32_t* col, const double* a,
-                          const double* b, double alpha, double beta, const double* d, const std::int64_t* dest,
+                          const double* b, const double* ab, const double* d, const std::int64_t* dest,
                           R* panels, FactorCounters* cnt) {
+  const double alpha = ab[0], beta = ab[1];
   double mx = 0.0;
   for (std::int64_t p = blockIdx.x * static_cast<std::int64_t>(blockDim.x) + threadIdx.x; p < nnz;
        p += static_cast<std::int64_t>(gridDim.x) * blockDim.x) {
@@ -116,7 +120,8 @@ __global__ void k_scatter(std::int64_t nnz, const std::int32_t* row, const std::
 // max |d_i d_j (alpha a_p + beta b_p)| alone (the null-pivot threshold of an inertia-only count,
 // whose entries are scattered level by level)
 __global__ void k_amax(std::int64_t nnz, const std::int32_t* row, const std::int32_t* col, const double* a,
-                       const double* b, double alpha, double beta, const double* d, FactorCounters* cnt) {
+                       const double* b, const double* ab, const double* d, FactorCounters* cnt) {
+  const double alpha = ab[0], beta = ab[1];
   double mx = 0.0;
   for (std::int64_t p = blockIdx.x * static_cast<std::int64_t>(blockDim.x) + threadIdx.x; p < nnz;
        p += static_cast<std::int64_t>(gridDim.x) * blockDim.x)
@@ -128,8 +133,9 @@ __global__ void k_amax(std::int64_t nnz, const std::int32_t* row, const std::int
 // panels[dest[p]] = d_i d_j (alpha a_p + beta b_p) for the listed entries p = idx[t] (one level's)
 template <class R>
 __global__ void k_scatter_list(const std::int64_t* idx, std::int64_t count, const std::int32_t* row,
-                               const std::int32_t* col, const double* a, const double* b, double alpha, double beta,
+                               const std::int32_t* col, const double* a, const double* b, const double* ab,
                                const double* d, const std::int64_t* dest, R* panels) {
+  const double alpha = ab[0], beta = ab[1];
   for (std::int64_t t = blockIdx.x * static_cast<std::int64_t>(blockDim.x) + threadIdx.x; t < count;
        t += static_cast<std::int64_t>(gridDim.x) * blockDim.x) {
     const std::int64_t p = idx[t];
@@ -1833,11 +1839,11 @@ void launch_zero_u64(unsigned long long* x, std::int64_t n, cudaStream_t s) {
 }
 
 void launch_scale_rowmax(std::int64_t nnz, const std::int32_t* row, const std::int32_t* col, const double* a,
-                         const double* b, double alpha, double beta, const double* d, unsigned long long* r,
+                         const double* b, const double* ab, const double* d, unsigned long long* r,
                          cudaStream_t s) {
   const int blocks = static_cast<int>(std::min<std::int64_t>((nnz + 255) / 256, 148 * 16));
   note_launches(1);
-  k_scale_rowmax<<<blocks, 256, 0, s>>>(nnz, row, col, a, b, alpha, beta, d, r);
+  k_scale_rowmax<<<blocks, 256, 0, s>>>(nnz, row, col, a, b, ab, d, r);
 }
 
 void launch_scale_update(std::int64_t n, double* d, unsigned long long* r, cudaStream_t s) {
@@ -1848,28 +1854,28 @@ void launch_scale_update(std::int64_t n, double* d, unsigned long long* r, cudaS
 
 template <class R>
 void launch_scatter(std::int64_t nnz, const std::int32_t* row, const std::int32_t* col, const double* a,
-                    const double* b, double alpha, double beta, const double* d, const std::int64_t* dest,
+                    const double* b, const double* ab, const double* d, const std::int64_t* dest,
                     R* panels, FactorCounters* cnt, cudaStream_t s) {
   const int blocks = static_cast<int>(std::min<std::int64_t>((nnz + 255) / 256, 148 * 16));
   note_launches(1);
-  k_scatter<R><<<blocks, 256, 0, s>>>(nnz, row, col, a, b, alpha, beta, d, dest, panels, cnt);
+  k_scatter<R><<<blocks, 256, 0, s>>>(nnz, row, col, a, b, ab, d, dest, panels, cnt);
 }
 
 void launch_amax(std::int64_t nnz, const std::int32_t* row, const std::int32_t* col, const double* a, const double* b,
-                 double alpha, double beta, const double* d, FactorCounters* cnt, cudaStream_t s) {
+                 const double* ab, const double* d, FactorCounters* cnt, cudaStream_t s) {
   const int blocks = static_cast<int>(std::min<std::int64_t>((nnz + 255) / 256, 148 * 16));
   note_launches(1);
-  k_amax<<<blocks, 256, 0, s>>>(nnz, row, col, a, b, alpha, beta, d, cnt);
+  k_amax<<<blocks, 256, 0, s>>>(nnz, row, col, a, b, ab, d, cnt);
 }
 
 template <class R>
 void launch_scatter_list(const std::int64_t* idx, std::int64_t count, const std::int32_t* row, const std::int32_t* col,
-                         const double* a, const double* b, double alpha, double beta, const double* d,
+                         const double* a, const double* b, const double* ab, const double* d,
                          const std::int64_t* dest, R* panels, cudaStream_t s) {
   if (count <= 0) return;
   const int blocks = static_cast<int>(std::min<std::int64_t>((count + 255) / 256, 148 * 16));
   note_launches(1);
-  k_scatter_list<R><<<blocks, 256, 0, s>>>(idx, count, row, col, a, b, alpha, beta, d, dest, panels);
+  k_scatter_list<R><<<blocks, 256, 0, s>>>(idx, count, row, col, a, b, ab, d, dest, panels);
 }
 
 template <class R>
@@ -1949,11 +1955,11 @@ cudaError_t launch_front_coop(const std::int32_t* list, const std::int32_t* cta_
 
 #define HSG_FACTOR_INSTANTIATE(R)                                                                                     \
   template void launch_scatter<R>(std::int64_t, const std::int32_t*, const std::int32_t*, const double*,             \
-                                  const double*, double, double, const double*, const std::int64_t*, R*,              \
+                                  const double*, const double*, const double*, const std::int64_t*, R*,              \
                                   FactorCounters*, cudaStream_t);                                                     \
   template void launch_zero_cb<R>(const std::int32_t*, int, int, const SnDev*, R*, cudaStream_t);                     \
   template void launch_scatter_list<R>(const std::int64_t*, std::int64_t, const std::int32_t*, const std::int32_t*,   \
-                                       const double*, const double*, double, double, const double*,                  \
+                                       const double*, const double*, const double*, const double*,                  \
                                        const std::int64_t*, R*, cudaStream_t);                                       \
   template void launch_extend_add<R>(const int2*, int, const SnDev*, const std::int32_t*, R*, R*, cudaStream_t);     \
   template void launch_front_small<R>(int, const std::int32_t*, int, const SnDev*, R*, R*, signed char*,              \

@@ -34,7 +34,7 @@ inline std::int64_t app_scratch_doubles(int m, int k) {
 void launch_fill(double* x, std::int64_t n, double v, cudaStream_t s);
 void launch_zero_u64(unsigned long long* x, std::int64_t n, cudaStream_t s);
 void launch_scale_rowmax(std::int64_t nnz, const std::int32_t* row, const std::int32_t* col, const double* a,
-                         const double* b, double alpha, double beta, const double* d, unsigned long long* r,
+                         const double* b, const double* ab, const double* d, unsigned long long* r,
                          cudaStream_t s);
 void launch_scale_update(std::int64_t n, double* d, unsigned long long* r, cudaStream_t s);
 // The front kernels are instantiated for R = double (the FP64 factorization that certifies inertia)
@@ -42,14 +42,14 @@ void launch_scale_update(std::int64_t n, double* d, unsigned long long* r, cudaS
 // contribution blocks hold R, the pivot scratch stays in units of doubles.
 template <class R>
 void launch_scatter(std::int64_t nnz, const std::int32_t* row, const std::int32_t* col, const double* a,
-                    const double* b, double alpha, double beta, const double* d, const std::int64_t* dest,
+                    const double* b, const double* ab, const double* d, const std::int64_t* dest,
                     R* panels, FactorCounters* cnt, cudaStream_t s);
 // inertia-only counts: the largest scaled entry alone, and the scatter of one level's entries
 void launch_amax(std::int64_t nnz, const std::int32_t* row, const std::int32_t* col, const double* a, const double* b,
-                 double alpha, double beta, const double* d, FactorCounters* cnt, cudaStream_t s);
+                 const double* ab, const double* d, FactorCounters* cnt, cudaStream_t s);
 template <class R>
 void launch_scatter_list(const std::int64_t* idx, std::int64_t count, const std::int32_t* row, const std::int32_t* col,
-                         const double* a, const double* b, double alpha, double beta, const double* d,
+                         const double* a, const double* b, const double* ab, const double* d,
                          const std::int64_t* dest, R* panels, cudaStream_t s);
 template <class R>
 void launch_zero_cb(const std::int32_t* list, int nlist, int chunks, const SnDev* sn, R* cb, cudaStream_t s);

@@ -5,6 +5,7 @@
 
 #include <cstdint>
 #include <memory>
+#include <functional>
 #include <mutex>
 #include <vector>
 
@@ -197,7 +198,10 @@ class GpuFactor {
   hsg_inertia_t run_factorization(double alpha, double beta, bool detection, bool shared, bool count_only);
   void run_numeric(double alpha, double beta, bool detection, bool count_only);
   template <class R>
-  void run_numeric_t(double alpha, double beta, bool detection, bool count_only);
+  void run_numeric_t(bool detection, bool count_only);
+  // captures `direct`'s work on stream_ into a graph (capture_mu_ held meanwhile); false where capturing
+  // is refused
+  bool capture(const std::function<void()>& direct, cudaGraphExec_t* exec, long long* launches);
   // forward, diagonal and backward sweeps of nr right-hand sides gathered in xwork (n x nr); with
   // graph, the launches are captured once per (xwork, vec, nr) in a CUDA graph and replayed
   void run_sweeps(double* xwork, double* vec, int nr, bool graph);
@@ -246,6 +250,7 @@ class GpuFactor {
   DevBuf<float> d_arena_f_;
   DevBuf<unsigned long long> d_r_;
   DevBuf<signed char> d_piv_;
+  DevBuf<double> d_ab_;  // (alpha, beta) of the factorization in flight
   DevBuf<FactorCounters> d_cnt_;
   DevBuf<int> d_level_done_;
   DevBuf<double> d_work_;
@@ -264,6 +269,23 @@ class GpuFactor {
     cudaGraphExec_t exec;
   };
   std::vector<SweepGraph> graphs_;
+  // captured factorizations by what their launches depend on beside the shift (which they read from
+  // pinned_): a form is captured at its second use (a single factorization would not win back the
+  // instantiation), valid until the plan or the buffers change
+  struct FactorGraph {
+    bool detection, count_only, shared;
+    const void* panels;
+    long long launches = 0;
+    cudaGraphExec_t exec = nullptr;
+  };
+  std::vector<FactorGraph> factor_graphs_;
+  bool factor_graphs_ok_ = true;  // false once a capture failed: launch directly
+  // pinned host memory that the factorization's transfers use: the shift in, the counters out
+  struct Pinned {
+    double ab[2];
+    FactorCounters cnt;
+  };
+  Pinned* pinned_ = nullptr;
   bool graphs_ok_ = true;  // false once a capture failed: launch directly
   // held while stream_ is capturing: another object's analyze_like synchronizes stream_, which is
   // not permitted during a capture
