@@ -21,7 +21,7 @@ constexpr int kRowChunk = (kAppDynDoubles - kRowStage) / kNB;  // rows staged at
 constexpr int kAppThreads = 256;
 constexpr int kCoopMinFront = 192;     // levels whose largest panel front is at least this use the cooperative kernel
 constexpr int kColsPerThread = kTile * kTile / kAppThreads;  // 16
-constexpr int kExtendAddCols = 8;      // contribution-block columns per extend-add CTA
+constexpr int kAssembleCols = 8;       // columns per assembly CTA (a warp each)
 // per-front scratch of the panel kernels (doubles): control block, two sets (alternate panels) of
 // block, original block, labels, pivot types and column maxima, backup of the panel's rows, W = L D
 // of the pending pivots (at most kKB, and at most the front's k)
@@ -52,10 +52,8 @@ void launch_scatter_list(const std::int64_t* idx, std::int64_t count, const std:
                          const double* a, const double* b, const double* ab, const double* d,
                          const std::int64_t* dest, R* panels, cudaStream_t s);
 template <class R>
-void launch_zero_cb(const std::int32_t* list, int nlist, int chunks, const SnDev* sn, R* cb, cudaStream_t s);
-template <class R>
-void launch_extend_add(const int2* items, int nitems, const SnDev* sn, const std::int32_t* rmap, R* panels, R* cb,
-                       cudaStream_t s);
+void launch_assemble(const int2* items, int nitems, const SnDev* sn, const std::int32_t* cptr, const int2* econt,
+                     const std::int32_t* rmap, R* panels, R* cb, cudaStream_t s);
 template <class R>
 void launch_front_small(int maxm, const std::int32_t* list, int nlist, const SnDev* sn, R* panels, R* cb,
                         signed char* piv, std::int32_t* pidx, const FactorParams& prm, FactorCounters* cnt,

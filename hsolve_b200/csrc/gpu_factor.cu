@@ -373,21 +373,21 @@ std::shared_ptr<FrontPlan> GpuFactor::make_plan() {
   std::int64_t w_total = 0;
   std::vector<std::int32_t> cptr;
   std::vector<ContribEntry> cent;
+  std::vector<int2> econt;
   std::vector<std::int32_t> lists;
   std::vector<int2> items;
   P.levels.assign(S.nlevels, LevelPlan{});
   std::int64_t scratch_max = 0;
   for (std::int32_t l = 0; l < S.nlevels; ++l) {
     LevelPlan& L = P.levels[l];
-    std::vector<std::int32_t> zero, s32, s64, app, all;
-    std::int64_t maxcb = 0, scratch = 0;
+    std::vector<std::int32_t> s32, s64, app, all;
+    std::int64_t scratch = 0;
     int maxm = 0;
     for (std::int32_t q = S.level_ptr[l]; q < S.level_ptr[l + 1]; ++q) {
       const std::int32_t s = S.level_sn[q];
       const int m = sn[s].m, k = sn[s].k;
       all.push_back(s);
       maxm = std::max(maxm, m);
-      if (m > k) { zero.push_back(s); maxcb = std::max<std::int64_t>(maxcb, static_cast<std::int64_t>(m - k) * (m - k)); }
       if (m <= 32) s32.push_back(s);
       else if (m <= kSmallMax) s64.push_back(s);
       else {
@@ -402,7 +402,6 @@ std::shared_ptr<FrontPlan> GpuFactor::make_plan() {
       cnt = static_cast<int>(v.size());
       lists.insert(lists.end(), v.begin(), v.end());
     };
-    put(zero, L.zero_off, L.zero_n);
     put(s32, L.s32_off, L.s32_n);
     put(s64, L.s64_off, L.s64_n);
     put(app, L.app_off, L.app_n);
@@ -436,6 +435,7 @@ std::shared_ptr<FrontPlan> GpuFactor::make_plan() {
         const std::int32_t base = static_cast<std::int32_t>(cent.size());
         for (int i = 0; i <= dw.m; ++i) cptr.push_back(base + num[i]);
         cent.resize(cent.size() + num[dw.m]);
+        econt.resize(cent.size());
         std::vector<std::int32_t> fill(num.begin(), num.end() - 1);
         for (std::int32_t e = S.child_ptr[sq]; e < S.child_ptr[sq + 1]; ++e) {
           const std::int32_t ch = S.children[e];
@@ -445,7 +445,9 @@ std::shared_ptr<FrontPlan> GpuFactor::make_plan() {
             ce.vec_off = sn[ch].vec_off;
             ce.a = a;
             ce.mc = mc;
-            cent[base + fill[S.rmap[S.rmap_off[ch] + a]]++] = ce;
+            const std::int32_t at = base + fill[S.rmap[S.rmap_off[ch] + a]]++;
+            cent[at] = ce;
+            econt[at] = make_int2(ch, a);
           }
         }
         dw.w_off = w_total;
@@ -578,25 +580,14 @@ std::shared_ptr<FrontPlan> GpuFactor::make_plan() {
       }
     }
     L.maxm = maxm;
-    L.zero_chunks = static_cast<int>(std::max<std::int64_t>(1, std::min<std::int64_t>(64, (maxcb + 4095) / 4096)));
-    // extend-add items by child rank
-    int maxrank = 0;
-    for (std::int32_t q = S.level_ptr[l]; q < S.level_ptr[l + 1]; ++q) {
-      const std::int32_t s = S.level_sn[q];
-      maxrank = std::max(maxrank, S.child_ptr[s + 1] - S.child_ptr[s]);
+    // assembly items: every front with children or a contribution block, eight columns a CTA (columns of
+    // the panel only where a child reaches them)
+    L.asm_off = static_cast<std::int64_t>(items.size());
+    for (std::int32_t s : all) {
+      const bool leaf = S.child_ptr[s] == S.child_ptr[s + 1];
+      for (int j0 = leaf ? sn[s].k : 0; j0 < sn[s].m; j0 += kAssembleCols) items.push_back(make_int2(s, j0));
     }
-    for (int r = 0; r < maxrank; ++r) {
-      const std::int64_t off = static_cast<std::int64_t>(items.size());
-      for (std::int32_t q = S.level_ptr[l]; q < S.level_ptr[l + 1]; ++q) {
-        const std::int32_t s = S.level_sn[q];
-        if (S.child_ptr[s] + r >= S.child_ptr[s + 1]) continue;
-        const std::int32_t c = S.children[S.child_ptr[s] + r];
-        const int mc = sn[c].m - sn[c].k;
-        for (int b0 = 0; b0 < mc; b0 += kExtendAddCols) items.push_back(make_int2(c, b0));
-      }
-      const int cnt = static_cast<int>(items.size() - off);
-      if (cnt) L.ea.push_back({off, cnt});
-    }
+    L.asm_n = static_cast<int>(static_cast<std::int64_t>(items.size()) - L.asm_off);
   }
   std::vector<std::int32_t> rows(S.rows.begin(), S.rows.end());
   {
@@ -651,6 +642,7 @@ std::shared_ptr<FrontPlan> GpuFactor::make_plan() {
   P.hcnt_total = hcnt_total;
   P.cptr.upload(cptr, stream_);
   P.cent.upload(cent, stream_);
+  P.econt.upload(econt, stream_);
   P.sbl.upload(sbl, stream_);
   P.tiles.upload(tiles, stream_);
   P.narrow.upload(narrow, stream_);
@@ -786,8 +778,7 @@ void GpuFactor::run_numeric_t(bool detection, bool count_only) {
       launch_scatter_list<R>(plan_->ent_idx.p + L.ent_off, L.ent_n, plan_->row.p, plan_->col.p, d_a_.p, d_b_.p, ab,
                              d_scale_.p, plan_->dest_cnt.p, panels, s);
     }
-    launch_zero_cb<R>(lists + L.zero_off, L.zero_n, L.zero_chunks, sn, cb, s);
-    for (const auto& ea : L.ea) launch_extend_add<R>(plan_->items.p + ea.first, ea.second, sn, plan_->rmap.p, panels, cb, s);
+    launch_assemble<R>(plan_->items.p + L.asm_off, L.asm_n, sn, plan_->cptr.p, plan_->econt.p, plan_->rmap.p, panels, cb, s);
     launch_front_small<R>(32, lists + L.s32_off, L.s32_n, sn, panels, cb, d_piv_.p, d_pidx_.p, prm, d_cnt_.p, d_failed_.p, s);
     launch_front_small<R>(kSmallMax, lists + L.s64_off, L.s64_n, sn, panels, cb, d_piv_.p, d_pidx_.p, prm, d_cnt_.p, d_failed_.p, s);
     if (shared_ ? L.coop_shared : L.coop) {

@@ -85,14 +85,13 @@ struct DevBuf {
 
 // Launch plan of one tree level of the fronts (built with the FrontPlan).
 struct LevelPlan {
-  std::int64_t zero_off = 0; int zero_n = 0; int zero_chunks = 1;
+  std::int64_t asm_off = 0; int asm_n = 0;  // assembly CTAs (FrontPlan::items)
   std::int64_t s32_off = 0; int s32_n = 0;
   std::int64_t s64_off = 0; int s64_n = 0;
   std::int64_t app_off = 0; int app_n = 0;
   bool coop = false;                 // large fronts: one cooperative launch, CTAs split by work
   std::int64_t cta_off = 0; int coop_ctas = 0; int done_slot = 0;
   std::int64_t all_off = 0; int all_n = 0; int maxm = 0;
-  std::vector<std::pair<std::int64_t, int>> ea;  // (offset into items, count) per child rank
   // solve sweeps: the level's CTA tasks (FrontPlan::tasks) of the forward and the backward sweep,
   // planned for launches of c + 1 column chunks; coop: some front has several CTAs (cooperative)
   std::int64_t fwd_task_off[2] = {0, 0}; int fwd_ctas[2] = {0, 0}; bool fwd_coop[2] = {false, false};
@@ -130,6 +129,7 @@ struct FrontPlan {
   DevBuf<std::int32_t> pfirst;     // per pivot: first column of its front
   DevBuf<std::int32_t> cptr;       // children's contributions per front position
   DevBuf<ContribEntry> cent;
+  DevBuf<int2> econt;              // the same contributions as (child, column of its contribution block)
   DevBuf<int2> sbl;                // wide super-blocks of the solve operators
   DevBuf<int4> tiles, narrow;
 };
