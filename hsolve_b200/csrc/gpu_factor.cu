@@ -674,6 +674,7 @@ void GpuFactor::alloc_work() {
   d_level_done_.alloc(static_cast<std::size_t>(std::max(1, P.ncoop)));
   d_work_.alloc(static_cast<std::size_t>(std::max<std::int64_t>(1, P.work_max)) * kSweepChunks);
   d_err_.alloc(1);
+  d_rhs_.alloc(1);
   d_sweep_cnt_.alloc(static_cast<std::size_t>(3 * std::max(1, sym_.ns) + P.hcnt_total) * kSweepChunks);
   w_ready_ = false;
 }
@@ -881,22 +882,17 @@ void GpuFactor::solve(double* b, std::int64_t nrhs, std::int64_t ldb, bool on_de
     db = d_btmp_.p;
     ld = n_;
   }
-  cuda_check(cudaMemsetAsync(d_err_.p, 0, sizeof(int), s), "reset solve status");
   cuda_check(cudaEventRecord(ev0_, s), "event");
   build_solve_operator();
-  launch_gather_scale(n_, nr, db, ld, d_scale_.p, plan_->iperm.p, d_xwork_.p, s);
-  run_sweeps(d_xwork_.p, d_vec_.p, nr, true);
-  launch_scatter_scale(n_, nr, db, ld, d_scale_.p, plan_->iperm.p, d_xwork_.p, s);
+  run_solve(db, ld, d_xwork_.p, d_vec_.p, nr, true);
   cuda_check(cudaEventRecord(ev1_, s), "event");
   cuda_check(cudaGetLastError(), "solve launch");
   if (!on_device) {
     cuda_check(cudaMemcpy2DAsync(b, ldb * sizeof(double), d_btmp_.p, n_ * sizeof(double), n_ * sizeof(double), nr,
                                  cudaMemcpyDeviceToHost, s), "D2H rhs");
   }
-  int err = 0;
-  cuda_check(cudaMemcpyAsync(&err, d_err_.p, sizeof(int), cudaMemcpyDeviceToHost, s), "solve status");
   cuda_check(cudaStreamSynchronize(s), "solve");
-  HSG_REQUIRE(err == 0, HSG_INTERNAL, "solve: a wait between the CTAs of a front timed out");
+  HSG_REQUIRE(pinned_->err == 0, HSG_INTERNAL, "solve: a wait between the CTAs of a front timed out");
   {
     float ms = 0.0f;
     cuda_check(cudaEventElapsedTime(&ms, ev0_, ev1_), "event time");
@@ -928,16 +924,11 @@ void GpuFactor::solve_with_scratch(double* b, std::int64_t nrhs, std::int64_t ld
   const int nr = static_cast<int>(nrhs);
   double* xwork = scratch;
   double* vec = scratch + static_cast<std::size_t>(n_) * nr;
-  cuda_check(cudaMemsetAsync(d_err_.p, 0, sizeof(int), s), "reset solve status");
   build_solve_operator();
-  launch_gather_scale(n_, nr, b, ldb, d_scale_.p, plan_->iperm.p, xwork, s);
-  run_sweeps(xwork, vec, nr, false);  // no graph: instantiating one may allocate
-  launch_scatter_scale(n_, nr, b, ldb, d_scale_.p, plan_->iperm.p, xwork, s);
+  run_solve(b, ldb, xwork, vec, nr, false);  // no graph: instantiating one may allocate
   cuda_check(cudaGetLastError(), "solve launch");
-  int err = 0;
-  cuda_check(cudaMemcpyAsync(&err, d_err_.p, sizeof(int), cudaMemcpyDeviceToHost, s), "solve status");
   cuda_check(cudaStreamSynchronize(s), "solve");
-  HSG_REQUIRE(err == 0, HSG_INTERNAL, "solve: a wait between the CTAs of a front timed out");
+  HSG_REQUIRE(pinned_->err == 0, HSG_INTERNAL, "solve: a wait between the CTAs of a front timed out");
 }
 
 void GpuFactor::clear_sweep_graphs() {
@@ -973,16 +964,23 @@ bool GpuFactor::capture(const std::function<void()>& direct, cudaGraphExec_t* ex
   return ok;
 }
 
-void GpuFactor::run_sweeps(double* xwork, double* vec, int nr, bool graph) {
+void GpuFactor::run_solve(double* b, std::int64_t ld, double* xwork, double* vec, int nr, bool graph) {
+  pinned_->rhs = SolveRhs{b, ld};
   auto direct = [&] {
+    cudaStream_t s = stream_;
+    cuda_check(cudaMemcpyAsync(d_rhs_.p, &pinned_->rhs, sizeof(SolveRhs), cudaMemcpyHostToDevice, s), "right-hand sides");
+    cuda_check(cudaMemsetAsync(d_err_.p, 0, sizeof(int), s), "reset solve status");
+    launch_gather_scale(n_, nr, d_rhs_.p, d_scale_.p, plan_->iperm.p, xwork, s);
     if (single()) run_sweeps_t<float>(xwork, vec, nr);
     else run_sweeps_t<double>(xwork, vec, nr);
+    launch_scatter_scale(n_, nr, d_rhs_.p, d_scale_.p, plan_->iperm.p, xwork, s);
+    cuda_check(cudaMemcpyAsync(&pinned_->err, d_err_.p, sizeof(int), cudaMemcpyDeviceToHost, s), "solve status");
   };
   if (!graph || !graphs_ok_) return direct();
   for (const SweepGraph& g : graphs_)
     if (g.xwork == xwork && g.vec == vec && g.nr == nr) {
       note_launches(g.launches);
-      cuda_check(cudaGraphLaunch(g.exec, stream_), "solve sweeps (graph)");
+      cuda_check(cudaGraphLaunch(g.exec, stream_), "solve (graph)");
       return;
     }
   // capture the sequence once; where capturing is refused (e.g. a cooperative launch), launch
@@ -995,7 +993,7 @@ void GpuFactor::run_sweeps(double* xwork, double* vec, int nr, bool graph) {
   }
   graphs_.push_back(SweepGraph{xwork, vec, nr, captured, exec});
   note_launches(captured);
-  cuda_check(cudaGraphLaunch(exec, stream_), "solve sweeps (graph)");
+  cuda_check(cudaGraphLaunch(exec, stream_), "solve (graph)");
 }
 
 template <class F>

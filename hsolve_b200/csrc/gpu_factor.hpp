@@ -14,6 +14,7 @@
 #include "common.hpp"
 #include "device.cuh"
 #include "hsg.h"
+#include "solve_kernels.cuh"
 #include "symbolic.hpp"
 
 namespace hsg {
@@ -202,9 +203,10 @@ class GpuFactor {
   // captures `direct`'s work on stream_ into a graph (capture_mu_ held meanwhile); false where capturing
   // is refused
   bool capture(const std::function<void()>& direct, cudaGraphExec_t* exec, long long* launches);
-  // forward, diagonal and backward sweeps of nr right-hand sides gathered in xwork (n x nr); with
-  // graph, the launches are captured once per (xwork, vec, nr) in a CUDA graph and replayed
-  void run_sweeps(double* xwork, double* vec, int nr, bool graph);
+  // solve of the nr right-hand sides at b (device, leading dimension ld): gather into xwork (n x nr),
+  // forward, diagonal and backward sweeps, scatter, status into pinned_; with graph, the launches are
+  // captured once per (xwork, vec, nr) in a CUDA graph and replayed (b and ld reach it through pinned_)
+  void run_solve(double* b, std::int64_t ld, double* xwork, double* vec, int nr, bool graph);
   void clear_sweep_graphs();
   template <class F>
   void run_sweeps_t(double* xwork, double* vec, int nr);
@@ -256,6 +258,7 @@ class GpuFactor {
   DevBuf<double> d_work_;
   // super-block solve operators of every front (built at the first solve after a factorization)
   DevBuf<double> d_w_;
+  DevBuf<SolveRhs> d_rhs_;
   DevBuf<int> d_err_;  // set by a solve sweep whose bounded wait ran out
   DevBuf<int> d_sweep_cnt_;       // per front: forward and backward publication counters, backward arrivals
   bool w_ready_ = false;
@@ -280,10 +283,13 @@ class GpuFactor {
   };
   std::vector<FactorGraph> factor_graphs_;
   bool factor_graphs_ok_ = true;  // false once a capture failed: launch directly
-  // pinned host memory that the factorization's transfers use: the shift in, the counters out
+  // pinned host memory that the transfers use: the shift in and the counters out of a factorization, the
+  // right-hand sides' place in and the status out of a solve
   struct Pinned {
     double ab[2];
     FactorCounters cnt;
+    SolveRhs rhs;
+    int err;
   };
   Pinned* pinned_ = nullptr;
   bool graphs_ok_ = true;  // false once a capture failed: launch directly

@@ -32,8 +32,11 @@ namespace hsg {
 
 namespace {
 
-__global__ void k_gather_scale(std::int64_t n, int nrhs, const double* b, std::int64_t ldb, const double* d,
+// the caller's right-hand sides are named in device memory, so that one captured solve serves them all
+__global__ void k_gather_scale(std::int64_t n, int nrhs, const SolveRhs* rhs, const double* d,
                                const std::int32_t* iperm, double* x) {
+  const double* b = rhs->b;
+  const std::int64_t ldb = rhs->ld;
   const std::int64_t total = n * nrhs;
   for (std::int64_t t = blockIdx.x * static_cast<std::int64_t>(blockDim.x) + threadIdx.x; t < total;
        t += static_cast<std::int64_t>(gridDim.x) * blockDim.x) {
@@ -42,8 +45,10 @@ __global__ void k_gather_scale(std::int64_t n, int nrhs, const double* b, std::i
   }
 }
 
-__global__ void k_scatter_scale(std::int64_t n, int nrhs, double* b, std::int64_t ldb, const double* d,
+__global__ void k_scatter_scale(std::int64_t n, int nrhs, const SolveRhs* rhs, const double* d,
                                 const std::int32_t* iperm, const double* x) {
+  double* b = rhs->b;
+  const std::int64_t ldb = rhs->ld;
   const std::int64_t total = n * nrhs;
   for (std::int64_t t = blockIdx.x * static_cast<std::int64_t>(blockDim.x) + threadIdx.x; t < total;
        t += static_cast<std::int64_t>(gridDim.x) * blockDim.x) {
@@ -849,20 +854,20 @@ __global__ void __launch_bounds__(256) k_bwd_tiny(const SolveTask* tasks, int nt
   }
 }
 
-void launch_gather_scale(std::int64_t n, int nrhs, const double* b, std::int64_t ldb, const double* d,
+void launch_gather_scale(std::int64_t n, int nrhs, const SolveRhs* rhs, const double* d,
                          const std::int32_t* iperm, double* x, cudaStream_t s) {
   const std::int64_t total = n * nrhs;
   const int blocks = static_cast<int>(std::min<std::int64_t>((total + 255) / 256, 148 * 16));
   note_launches(1);
-  k_gather_scale<<<blocks, 256, 0, s>>>(n, nrhs, b, ldb, d, iperm, x);
+  k_gather_scale<<<blocks, 256, 0, s>>>(n, nrhs, rhs, d, iperm, x);
 }
 
-void launch_scatter_scale(std::int64_t n, int nrhs, double* b, std::int64_t ldb, const double* d,
+void launch_scatter_scale(std::int64_t n, int nrhs, const SolveRhs* rhs, const double* d,
                           const std::int32_t* iperm, const double* x, cudaStream_t s) {
   const std::int64_t total = n * nrhs;
   const int blocks = static_cast<int>(std::min<std::int64_t>((total + 255) / 256, 148 * 16));
   note_launches(1);
-  k_scatter_scale<<<blocks, 256, 0, s>>>(n, nrhs, b, ldb, d, iperm, x);
+  k_scatter_scale<<<blocks, 256, 0, s>>>(n, nrhs, rhs, d, iperm, x);
 }
 
 template <class F>

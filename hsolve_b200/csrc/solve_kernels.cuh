@@ -8,9 +8,15 @@
 
 namespace hsg {
 
-void launch_gather_scale(std::int64_t n, int nrhs, const double* b, std::int64_t ldb, const double* d,
+// right-hand sides of a solve: column-major, leading dimension ld
+struct SolveRhs {
+  double* b;
+  std::int64_t ld;
+};
+
+void launch_gather_scale(std::int64_t n, int nrhs, const SolveRhs* rhs, const double* d,
                          const std::int32_t* iperm, double* x, cudaStream_t s);
-void launch_scatter_scale(std::int64_t n, int nrhs, double* b, std::int64_t ldb, const double* d,
+void launch_scatter_scale(std::int64_t n, int nrhs, const SolveRhs* rhs, const double* d,
                           const std::int32_t* iperm, const double* x, cudaStream_t s);
 
 // The kernels below that read the factor are instantiated for F = double (FP64 factors) and
