@@ -1368,11 +1368,11 @@ __device__ void app_restore(AppFront<R>& F, const StepView& v, int rank, int nr,
 // Blocked step. The pivots [fb, p + q) eliminated since the last full update are pending: their
 // Schur update has reached only the panels factorized since. After a panel the pending update goes
 // either to the whole trailing matrix (a flush: the panel rejected columns, the candidate range
-// ends, or kKB pivots would be pending after the next panel) or to the next panel's columns only.
+// ends, or more than pending_max(m) pivots would be pending after the next panel) or to the next panel's columns only.
 // A column is therefore up to date when its panel is factorized, and every other trailing column
-// receives the pending pivots in one rank-(<= kKB) update instead of one update per panel.
-__device__ __forceinline__ bool app_flushes(int p, int w, int q, int lim, int fb) {
-  return q < w || p + q >= lim || p + q + kNB - fb > kKB;
+// receives the pending pivots in one rank-(<= pending_max(m)) update instead of one update per panel.
+__device__ __forceinline__ bool app_flushes(int m, int p, int w, int q, int lim, int fb) {
+  return q < w || p + q >= lim || p + q + kNB - fb > pending_max(m);
 }
 
 // All ranks: C(i, c) -= sum_{s in [fb, p+q)} L(i, s) W(c, s), W = L D, over the lower triangle
@@ -1411,7 +1411,7 @@ __device__ void app_update(AppFront<R>& F, const StepView& v, int rank, int nr, 
   const int K = from - fb;
   const int rows = m - from;
   if (rows <= 0 || K <= 0) return;
-  const bool flush = app_flushes(p, w, q, lim, fb);
+  const bool flush = app_flushes(m, p, w, q, lim, fb);
   const int col_hi = flush ? m : min(m, from + min(kNB, lim - from));
   const int rej_hi = flush && q < w ? p + w : 0;  // columns below this take only the pivots >= p
   const int nt = (rows + kTile - 1) / kTile;
@@ -1618,7 +1618,7 @@ __device__ void app_advance(AppFront<R>& F, int q, bool moved) {
   const int p = c->p, w = c->w;
   const int np = p + q, r = w - q;
   const int lim = c->lim;
-  const bool flushed = app_flushes(p, w, q, lim, c->fb);
+  const bool flushed = app_flushes(F.f.m, p, w, q, lim, c->fb);
   if (r > 0 && np + r < lim && !moved) {
     for (int t = 0; t < r; ++t) {
       front_swap(F.f, np + t, lim - r + t, F.plab);
@@ -1661,6 +1661,7 @@ __device__ void app_next_block(AppFront<R>& F, const StepView& v, int slot, cons
   const int Kpad = (K + 7) & ~7;
   set_slot(F, slot);
   R* Ls = stage;
+  static_assert(2 * kKB * kLd <= kAppDynDoubles, "the pending pivots' rows fit the staging area");
   R* Ws = stage + kKB * kLd;
   __syncthreads();  // the staging area's last users are done
   for (int s = warp; s < Kpad; s += kAppThreads / 32) {
@@ -1683,7 +1684,7 @@ __device__ void app_next_block(AppFront<R>& F, const StepView& v, int slot, cons
     c->prog = 1;
     c->force = 0;
     c->stop = 0;
-    if (app_flushes(v.p, v.w, v.w, v.lim, fb)) c->fb = p;
+    if (app_flushes(m, v.p, v.w, v.w, v.lim, fb)) c->fb = p;
     bk_begin(sm.bst, w);
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");

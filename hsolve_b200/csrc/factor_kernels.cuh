@@ -11,7 +11,17 @@ namespace hsg {
 constexpr int kSmallMax = 64;          // fronts up to this order are factorized in shared memory
 constexpr int kNB = 32;                // panel width of the a-posteriori pivoting kernel
 constexpr int kTile = 64;              // trailing-update tile (rows = cols)
-constexpr int kKB = 128;               // pending pivots whose trailing update is applied at once (blocked step)
+// Pending pivots whose trailing update is applied at once (blocked step). More of them spread a tile's fixed
+// costs and its pass over C over more products, but lengthen the next panel's own updates, which are on
+// the chain: n = 291,359 (fronts to 5,861) 53.7 ms a factorization with 128, 52.3 with 192, 51.9 with 224;
+// n = 21,660 (fronts to 1,279) 2.61, 2.63, 2.65. With 224 from an order of 1,400 on: 51.8 and 2.61 ms, from
+// 2,048 on 52.2, from 3,000 on 52.2.
+constexpr int kKB = 224;               // most of any front
+constexpr int kKBLargeFront = 1400;
+#if defined(__CUDACC__)
+__host__ __device__
+#endif
+inline int pending_max(int m) { return m >= kKBLargeFront ? kKB : 128; }
 constexpr int kUpdLd = kTile + 4;      // column stride of the staged update operands (conflict-free fragment reads)
 constexpr int kUpdChunk = 32;          // pivots of a tile's operands staged at once
 constexpr int kUpdStages = 4;          // staged chunks (one computed, the others in flight)
@@ -24,11 +34,11 @@ constexpr int kColsPerThread = kTile * kTile / kAppThreads;  // 16
 constexpr int kAssembleCols = 8;       // columns per assembly CTA (a warp each)
 // per-front scratch of the panel kernels (doubles): control block, two sets (alternate panels) of
 // block, original block, labels, pivot types and column maxima, backup of the panel's rows, W = L D
-// of the pending pivots (at most kKB, and at most the front's k)
+// of the pending pivots (at most pending_max, and at most the front's k)
 constexpr int kAppCtrlDoubles = 8;
 constexpr int kAppSlotDoubles = 2 * kNB * kNB + kNB / 2 + kNB / 8 + 2 * kNB;
 inline std::int64_t app_scratch_doubles(int m, int k) {
-  return kAppCtrlDoubles + 2 * kAppSlotDoubles + static_cast<std::int64_t>(m) * (kNB + (k < kKB ? k : kKB));
+  return kAppCtrlDoubles + 2 * kAppSlotDoubles + static_cast<std::int64_t>(m) * (kNB + (k < pending_max(m) ? k : pending_max(m)));
 }
 
 void launch_fill(double* x, std::int64_t n, double v, cudaStream_t s);

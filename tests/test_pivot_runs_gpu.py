@@ -53,6 +53,13 @@ def test_one_dense_front(kind, n):
     _check(_dense(kind, n, rng))
 
 
+@pytest.mark.parametrize("kind", ["runs", "mixed"])
+@pytest.mark.parametrize("n", [1399, 1400, 1457])
+def test_pending_pivots_of_large_fronts(kind, n):
+    """Fronts of 1,400 rows and more keep 224 pivots pending instead of 128."""
+    _check(_dense(kind, n, np.random.default_rng(n)))
+
+
 @pytest.mark.parametrize("kind", ["runs", "pairs", "mixed"])
 @pytest.mark.parametrize("k,c", [(1, 31), (5, 28), (31, 33), (32, 32), (33, 31), (40, 60), (64, 33), (70, 130)])
 def test_fronts_with_contribution_rows(kind, k, c):
