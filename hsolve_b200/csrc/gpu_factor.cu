@@ -697,9 +697,14 @@ std::size_t GpuFactor::factor_bytes() const {
   return el * (d_panels_.n + d_panels_f_.n + d_w_.n + d_w_f_.n);
 }
 
-// The launches of a factorization are queued from one graph after its first use of a form: 50 to 120
-// launches at 5.3 us of host time each, 0.6 to 1.1 us in a graph, bound the small factorizations (a count at
-// n = 737: 492 us, now 379; a factorization at n = 3,021: 770, now 650).
+// The launches of a small factorization are queued from one graph once a form has been used kGraphUses
+// times: 50 to 120 launches at 5.3 us of host time each, 0.6 to 1.1 us in a graph, bound it (a count at
+// n = 737: 492 us, 379 from the graph; a factorization at n = 3,021: 770 and 650). Capturing and
+// instantiating costs 2 to 3 ms once, so that a few factorizations would not win it back, and above
+// kGraphOrder the launches hide behind the kernels (n = 109,744: 12.4 and 12.3 ms).
+constexpr int kGraphUses = 8;
+constexpr std::int64_t kGraphOrder = 65536;
+
 void GpuFactor::run_numeric(double alpha, double beta, bool detection, bool count_only) {
   pinned_->ab[0] = alpha;
   pinned_->ab[1] = beta;
@@ -712,12 +717,13 @@ void GpuFactor::run_numeric(double alpha, double beta, bool detection, bool coun
     if (single()) run_numeric_t<float>(detection, count_only);
     else run_numeric_t<double>(detection, count_only);
   };
-  if (!factor_graphs_ok_) return direct();
+  if (!factor_graphs_ok_ || n_ > kGraphOrder) return direct();
   const void* panels = single() ? static_cast<const void*>(count_only ? d_arena_f_.p : d_panels_f_.p)
                                 : static_cast<const void*>(count_only ? d_arena_.p : d_panels_.p);
   FactorGraph* g = nullptr;
   for (FactorGraph& f : factor_graphs_)
     if (f.detection == detection && f.count_only == count_only && f.shared == shared_ && f.panels == panels) g = &f;
+  if (g && !g->exec && ++g->uses < kGraphUses) return direct();
   if (!g) {
     FactorGraph f;
     f.detection = detection;

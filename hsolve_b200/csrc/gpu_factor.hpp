@@ -273,11 +273,12 @@ class GpuFactor {
   };
   std::vector<SweepGraph> graphs_;
   // captured factorizations by what their launches depend on beside the shift (which they read from
-  // pinned_): a form is captured at its second use (a single factorization would not win back the
-  // instantiation), valid until the plan or the buffers change
+  // pinned_), once a form has been used often enough to win the capture back; valid until the plan or the
+  // buffers change
   struct FactorGraph {
     bool detection, count_only, shared;
     const void* panels;
+    int uses = 1;
     long long launches = 0;
     cudaGraphExec_t exec = nullptr;
   };
