@@ -394,20 +394,7 @@ __device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1, double a, do
                : "+d"(d0), "+d"(d1) : "d"(a), "d"(b));
 }
 
-// 1 / d for normal d away from the ends of the exponent range: the hardware's approximation and
-// Newton's iteration r += r (1 - d r). Without the range branches of a division, the pivot chain below
-// can be scheduled around it.
-__device__ __forceinline__ double rcp_newton(double d) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  double e = fma(-d, r, 1.0);
-  e = fma(e, e, e);
-  r = fma(e, r, r);
-  e = fma(-d, r, 1.0);
-  return fma(e, r, r);
-}
-__device__ __forceinline__ float rcp_newton(float d) { return 1.0f / d; }
-constexpr double kRcpMin = 1e-280, kRcpMax = 1e280;  // |d| that rcp_newton is used for
+constexpr double kRcpMin = 1e-280, kRcpMax = 1e280;  // |d| whose reciprocal is away from the ends of the range
 
 // The bits of |v| that order like the values (the upper word of a double), and a bound of every
 // value with those bits.
@@ -463,8 +450,7 @@ struct __align__(16) QuadSmem {
 // Ends at st.lim or before the first column whose test fails.
 //
 // A pivot is a chain of dependent operations (1 / d, scale, update, the next d), not work. A 32 x 32
-// block takes 7,700 cycles; with one warp for the whole block it took 36,100, with one pivot a
-// barrier 12,800.
+// block takes 9,500 cycles: 16,900 with every row divided by d, 36,100 with one warp for the whole block.
 template <int MAXM, int NT, class R>
 __device__ __forceinline__ void fast_pivots(RegTri<MAXM, NT, R>& y, QuadSmem<MAXM, R>& sm, R* F, int ld, double u,
                                             double thr, signed char* pv, StepShared& st) {
@@ -498,7 +484,7 @@ __device__ __forceinline__ void fast_pivots(RegTri<MAXM, NT, R>& y, QuadSmem<MAX
       double gc[4];
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
-        const R inv = rcp_newton(a[t][t]);
+        const R inv = R(1) / a[t][t];
         R la[4];
 #pragma unroll
         for (int s = t + 1; s < 4; ++s) la[s] = a[t][s] * inv;
