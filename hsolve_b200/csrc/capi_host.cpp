@@ -14,9 +14,14 @@ namespace hsg {
 namespace {
 thread_local std::string g_last_error;
 std::atomic<long long> g_launches{0};
+thread_local long long t_launches = 0;
 }  // namespace
 void set_last_error(const std::string& msg) { g_last_error = msg; }
-void note_launches(long long count) { g_launches.fetch_add(count, std::memory_order_relaxed); }
+void note_launches(long long count) {
+  g_launches.fetch_add(count, std::memory_order_relaxed);
+  t_launches += count;
+}
+long long thread_launches() { return t_launches; }
 }  // namespace hsg
 
 using namespace hsg;

@@ -35,6 +35,8 @@ void set_last_error(const std::string& msg);
 
 // Kernel launches issued by this library (exported as hsg_kernel_launches).
 void note_launches(long long count);
+// Those of the calling thread (what a capture by this thread counts, whatever other threads launch).
+long long thread_launches();
 
 // Runs f(), mapping exceptions to status codes and recording the message (C ABI wrapper).
 template <class F>

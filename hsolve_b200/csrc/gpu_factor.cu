@@ -946,7 +946,7 @@ void GpuFactor::clear_sweep_graphs() {
 }
 
 bool GpuFactor::capture(const std::function<void()>& direct, cudaGraphExec_t* exec, long long* launches) {
-  const long long l0 = hsg_kernel_launches();
+  const long long l0 = thread_launches();
   cudaGraph_t cg = nullptr;
   std::unique_lock<std::mutex> lk(capture_mu_);
   bool ok = cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
@@ -961,7 +961,7 @@ bool GpuFactor::capture(const std::function<void()>& direct, cudaGraphExec_t* ex
     if (cg) cudaGraphDestroy(cg);
   }
   lk.unlock();
-  *launches = hsg_kernel_launches() - l0;
+  *launches = thread_launches() - l0;
   note_launches(-*launches);  // counted when the graph runs
   if (!ok) {
     cudaGetLastError();  // the failed capture's error is not sticky
