@@ -36,6 +36,11 @@ class _Estimate(ctypes.Structure):
                 ("max_front", ctypes.c_int32), ("ordering_s", ctypes.c_double), ("analyze_s", ctypes.c_double)]
 
 
+class _GraphStats(ctypes.Structure):
+    _fields_ = [("factor_graphs", ctypes.c_int64), ("factor_replays", ctypes.c_int64),
+                ("solve_graphs", ctypes.c_int64), ("solve_replays", ctypes.c_int64)]
+
+
 # hs::Error::Code names in status order (status = code + 1), include/hsolve/error.hpp:16-26
 STATUS_NAMES = {0: "ok", 1: "invalid_input", 2: "io", 3: "not_hermitian", 4: "unsupported",
                 5: "factorization_failed", 6: "singular", 7: "out_of_memory_budget", 8: "not_converged",
@@ -65,6 +70,7 @@ SIGNATURES = {
     "hsg_set_null_pivot_detection": (ctypes.c_int, [_P, _I32]),
     "hsg_pivot_order": (ctypes.c_int, [_P, _P]),
     "hsg_order": (_I64, [_P]),
+    "hsg_graph_stats": (ctypes.c_int, [_P, _P]),
     "hsg_clear_analysis_cache": (ctypes.c_int, []),
     "hsg_spmm": (ctypes.c_int, [_I64, _P, _P, _P, _P, _I64, _P, _I64, _I64, _D, _D]),
     "hsg_shifted_residual": (ctypes.c_int, [_I64, _P, _P, _P, _P, _P, _P, _D, _P, _I64, _P, _I64, _P, _I64, _I64,
@@ -228,6 +234,12 @@ class Factorization:
 
     def order(self) -> int:
         return int(lib().hsg_order(self._h))
+
+    def graph_stats(self) -> dict:
+        """Graphs held and calls replayed from them (hsg_graph_stats)."""
+        s = _GraphStats()
+        check(lib().hsg_graph_stats(self._h, ctypes.byref(s)))
+        return {f: getattr(s, f) for f, _ in _GraphStats._fields_}
 
 
 def csr_inspect(m):

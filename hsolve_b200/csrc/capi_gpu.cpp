@@ -115,6 +115,13 @@ int hsg_pivot_order(const hsg_factor* f, int32_t* out) {
   });
 }
 
+int hsg_graph_stats(const hsg_factor* f, hsg_graph_stats_t* out) {
+  return guarded([&] {
+    HSG_REQUIRE(out, HSG_INVALID_INPUT, "hsg_graph_stats: null output");
+    *out = get(f).graph_stats();
+  });
+}
+
 int hsg_clear_analysis_cache(void) {
   return guarded([] { clear_analysis_cache(); });
 }

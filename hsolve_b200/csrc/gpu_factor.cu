@@ -738,6 +738,7 @@ void GpuFactor::run_numeric(double alpha, double beta, bool detection, bool coun
     return direct();
   }
   note_launches(g->launches);
+  ++factor_replays_;
   cuda_check(cudaGraphLaunch(g->exec, stream_), "factorization (graph)");
 }
 
@@ -986,6 +987,7 @@ void GpuFactor::run_solve(double* b, std::int64_t ld, double* xwork, double* vec
   for (const SweepGraph& g : graphs_)
     if (g.xwork == xwork && g.vec == vec && g.nr == nr) {
       note_launches(g.launches);
+      ++solve_replays_;
       cuda_check(cudaGraphLaunch(g.exec, stream_), "solve (graph)");
       return;
     }
@@ -999,7 +1001,17 @@ void GpuFactor::run_solve(double* b, std::int64_t ld, double* xwork, double* vec
   }
   graphs_.push_back(SweepGraph{xwork, vec, nr, captured, exec});
   note_launches(captured);
+  ++solve_replays_;
   cuda_check(cudaGraphLaunch(exec, stream_), "solve (graph)");
+}
+
+hsg_graph_stats_t GpuFactor::graph_stats() const {
+  hsg_graph_stats_t s{};
+  for (const FactorGraph& g : factor_graphs_) s.factor_graphs += g.exec != nullptr;
+  s.factor_replays = factor_replays_;
+  s.solve_graphs = static_cast<std::int64_t>(graphs_.size());
+  s.solve_replays = solve_replays_;
+  return s;
 }
 
 template <class F>

@@ -190,6 +190,7 @@ class GpuFactor {
   };
   const DeviceStats& device_stats() const { return dstats_; }
   void reset_device_stats() { dstats_ = DeviceStats{}; }
+  hsg_graph_stats_t graph_stats() const;
 
  private:
   // plan_ = a new plan of sym_ (make_plan) and the per-object work arrays sized for it
@@ -272,6 +273,7 @@ class GpuFactor {
     cudaGraphExec_t exec;
   };
   std::vector<SweepGraph> graphs_;
+  long long factor_replays_ = 0, solve_replays_ = 0;
   // captured factorizations by what their launches depend on beside the shift (which they read from
   // pinned_), once a form has been used often enough to win the capture back; valid until the plan or the
   // buffers change

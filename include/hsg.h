@@ -160,6 +160,14 @@ HSG_API int hsg_pivot_order(const hsg_factor* f, int32_t* out);
 /* SparseFactorization::order() (factor.hpp:441-442). */
 HSG_API int64_t hsg_order(const hsg_factor* f);
 
+/* Captured work of a handle since its creation (instrumentation; no counterpart in hsolve): the graphs it holds,
+ * and the factorizations (counts among them) and solves that were replayed from one. */
+typedef struct {
+  int64_t factor_graphs, factor_replays;
+  int64_t solve_graphs, solve_replays;
+} hsg_graph_stats_t;
+HSG_API int hsg_graph_stats(const hsg_factor* f, hsg_graph_stats_t* out);
+
 /* Empties the process-wide cache of nested-dissection analyses (keyed by sparsity pattern), so that
  * the next analysis of any pattern runs the ordering and the symbolic factorization again; handles
  * that already hold an analysis keep it (instrumentation for cold-call timing; no counterpart in
