@@ -1089,7 +1089,11 @@ hsg_estimate_t GpuFactor::estimate() const {
   e.nnz_l = sym_.nnz_l;
   e.flops = sym_.flops;
   const double el = single() ? 4.0 : 8.0;  // bytes of a factor entry
-  e.device_mb = (el * static_cast<double>(sym_.factor_entries + sym_.cb_arena) + 8.0 * static_cast<double>(4 * nnz_ + 4 * n_)) / 1e6;
+  // factors and contribution blocks, the pencil, the pivoting scratch of the widest level (in large fronts up to
+  // 256 columns of the front) and the fronts' contribution lists
+  const double contributions = static_cast<double>(plan_->cent.n) * (sizeof(ContribEntry) + sizeof(int2));
+  e.device_mb = (el * static_cast<double>(sym_.factor_entries + sym_.cb_arena) + 8.0 * static_cast<double>(4 * nnz_ + 4 * n_) +
+                 8.0 * static_cast<double>(plan_->scratch_max) + contributions) / 1e6;
   e.supernodes = sym_.ns;
   e.levels = sym_.nlevels;
   e.max_front = sym_.max_front;
