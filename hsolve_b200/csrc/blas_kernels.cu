@@ -6,6 +6,7 @@
 //    Y = beta Y + alpha X S for the block Gram-Schmidt / CholQR updates and Ritz vectors
 //    (BlockOrthonormalizer, src/eigen/block_ortho.cpp:165,270; orthogonalize_block_cgs2,
 //    src/linalg/dense_ops.hpp:180).
+#include <algorithm>
 #include <cstdint>
 #include <mutex>
 
@@ -21,29 +22,58 @@ void cuda_check(cudaError_t e, const char* what);
 
 namespace {
 
-// Rows of a CSR product are summed by four lanes each, eight rows a warp: the entries of a row are read
-// by neighbouring lanes, the gathers of neighbouring rows fall into the same lines, and the partial
-// sums take two shuffle steps. A curl-curl row has at most 13 entries: a warp per row left 19 lanes idle
-// and spent most of its time in five-step reductions (the residual of 8 columns at n = 21,660: 122 us,
-// now 11). Rows of more than kLongRow entries are summed by the whole warp.
-constexpr int kLongRow = 128;
+// Rows of a CSR product: a CTA takes a chunk of 64 rows (16 where the matrix has few) and sums each by four
+// lanes: the entries of a row are read by neighbouring lanes, the gathers of neighbouring rows fall into the same
+// lines, and the partial sums take two shuffle steps. A curl-curl row has at most 13 entries: a warp per row left
+// 19 lanes idle and spent most of its time in five-step reductions (the call for the residual of 8 columns at
+// n = 21,660: 135 us, now 24).
+//
+// Longer rows want more lanes: chunks above most_entries a row take sixteen lanes a row, rows above kLongRow a
+// warp each. With four lanes up to 128 entries and the warp's own eight rows one after another above, the
+// residual of 8 columns took 33 us at n = 3,000 with 64 entries a row (now 25; a warp per row 41), 112 with 192
+// entries (39; 56) and 1,104 where 8 of the 3,000 rows were full (162; 215); a product of 8 columns 524 us there
+// (67; 95).
+constexpr int kRowThreads = 256;
+constexpr int kRowWarps = kRowThreads / 32;
+constexpr int kChunk = kRowThreads / 4, kSmallChunk = kRowThreads / 16;
+constexpr int kSmallRows = 444 * kSmallChunk;  // 16 lanes a row fill three CTAs an SM
+constexpr int kLongRow = 512;
 
-// f(value, column) for this lane's entries of row i (quad: every 4th; rows beyond kLongRow are left to
-// the warp). Four entries are read ahead of their gathers: a curl-curl row is one round of latencies.
-template <class Fn>
-__device__ __forceinline__ void quad_entries(const std::int64_t* rp, const std::int32_t* ci, const double* v,
-                                             std::int64_t i, bool in, Fn&& f) {
-  constexpr int kAhead = 4;
-  const int sub = threadIdx.x & 3;
-  const std::int64_t q0 = in ? rp[i] : 0, q1 = in ? rp[i + 1] : 0;
-  if (q1 - q0 > kLongRow) return;
-  for (std::int64_t q = q0 + sub; q < q1; q += 4 * kAhead) {
+// Entries a row up to which a chunk takes four lanes a row. In few rows they leave the device idle (n = 3,000,
+// residual of 8 columns, four and sixteen lanes: 13 entries 22 and 20 us, 30 entries 28 and 21; one column
+// 17.4 and 18.4, 17.3 and 17.7); in many rows they move less (n = 100,000, 8 columns, 96 entries: 188 and
+// 308 us, 128 entries 231 and 397; a product of one column 43 and 39, 52 and 44).
+template <int P>
+__device__ __forceinline__ int most_entries(int chunk) {
+  return chunk == kSmallChunk ? 24 : (P == 1 ? 96 : 128);
+}
+
+// f(value, column) for this lane's entries of the row [q0, q1): every G-th, kAhead of them read before the
+// gathers (a curl-curl row is one round of latencies).
+template <int G, int kAhead, bool kWhole, class Fn>
+__device__ __forceinline__ void group_entries(std::int64_t q0, std::int64_t q1, const std::int32_t* ci, const double* v,
+                                              Fn&& f) {
+  std::int64_t q = q0 + (threadIdx.x & (G - 1));
+  if constexpr (G > 4 && kWhole) {  // (rows of many rounds: the whole ones without tests)
+    for (; q + G * (kAhead - 1) < q1; q += G * kAhead) {
+      double a[kAhead];
+      std::int32_t j[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        a[u] = v[q + G * u];
+        j[u] = ci[q + G * u];
+      }
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) f(a[u], j[u]);
+    }
+  }
+  for (; q < q1; q += G * kAhead) {
     double a[kAhead];
     std::int32_t j[kAhead];
 #pragma unroll
     for (int u = 0; u < kAhead; ++u) {
-      a[u] = q + 4 * u < q1 ? v[q + 4 * u] : 0.0;
-      j[u] = q + 4 * u < q1 ? ci[q + 4 * u] : -1;
+      a[u] = q + G * u < q1 ? v[q + G * u] : 0.0;
+      j[u] = q + G * u < q1 ? ci[q + G * u] : -1;
     }
 #pragma unroll
     for (int u = 0; u < kAhead; ++u)
@@ -51,87 +81,162 @@ __device__ __forceinline__ void quad_entries(const std::int64_t* rp, const std::
   }
 }
 
-// The quad's sums of P columns, scattered: lane sub keeps columns quad_col<P>() .. + P / 4 (P < 4: one
-// column, held by several lanes) in a[0 ..]; half the shuffles of a full reduction per step.
-template <int P>
-__device__ __forceinline__ void quad_scatter(double (&a)[P]) {
-  int width = P;
+// The G lanes' sums of P columns, scattered: a lane keeps columns first .. first + kCols in a[0 ..] (several
+// lanes the same column where P < G: `writer` is one of them); a halving of the columns a step while there
+// are columns to halve, which is half the shuffles of a full reduction.
+constexpr int log2i(int v) { return v <= 1 ? 0 : 1 + log2i(v / 2); }
+template <int P, int G>
+struct GroupCols {
+  static constexpr int kHalvings = log2i(P) < log2i(G) ? log2i(P) : log2i(G);
+  static constexpr int kCols = P >> kHalvings, kShare = G >> kHalvings;
+  int first;
+  bool writer;
+  __device__ __forceinline__ GroupCols() {
+    const int sub = threadIdx.x & (G - 1);
+    first = sub / kShare * kCols;
+    writer = sub % kShare == 0;
+  }
+  __device__ __forceinline__ static void sum(double (&a)[P]) {
+    int width = P;
 #pragma unroll
-  for (int o = 2; o > 0; o >>= 1) {
-    const bool up = (threadIdx.x & o) != 0;
-    if (width > 1) {
-      width /= 2;
+    for (int o = G / 2; o > 0; o >>= 1) {
+      const bool up = (threadIdx.x & o) != 0;
+      if (width > 1) {
+        width /= 2;
 #pragma unroll
-      for (int c = 0; c < P / 2; ++c)
-        if (c < width) {
-          const double send = up ? a[c] : a[c + width], keep = up ? a[c + width] : a[c];
-          a[c] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-    } else {
-      a[0] += __shfl_xor_sync(0xffffffffu, a[0], o);
+        for (int c = 0; c < P / 2; ++c)
+          if (c < width) {
+            const double send = up ? a[c] : a[c + width], keep = up ? a[c + width] : a[c];
+            a[c] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+          }
+      } else {
+        a[0] += __shfl_xor_sync(0xffffffffu, a[0], o);
+      }
     }
   }
-}
-template <int P>
-__device__ __forceinline__ int quad_col() {
-  const int sub = threadIdx.x & 3;
-  return P >= 4 ? sub * (P / 4) : (P == 2 ? sub >> 1 : 0);
-}
+};
 
-// the warp's long rows, one after another: f(row, owner) with the row's quad `owner`
-template <class Fn>
-__device__ __forceinline__ void long_rows(const std::int64_t* rp, std::int64_t row0, std::int64_t n, Fn&& f) {
-  const int lane = threadIdx.x & 31;
-  const std::int64_t i = row0 + (lane >> 2);
-  unsigned m = __ballot_sync(0xffffffffu, (lane & 3) == 0 && i < n && rp[i + 1] - rp[i] > kLongRow);
-  while (m) {
-    const int o = __ffs(m) - 1;
-    m &= m - 1;
-    f(row0 + (o >> 2), o >> 2);
+// The rows of a matrix, chunk by chunk: quad(i, span(i, end)) for this lane's row i of a chunk that ends at `end`,
+// by four lanes (i may lie beyond), or wide(row0, end) for a chunk of many entries; entries(a, b) are those of the
+// rows [a, b). Both leave out the long rows, which take a warp each, long_row(i): a CTA's warps share those of
+// eight groups spread over the matrix, so that neighbouring long rows meet as many CTAs as there are groups of
+// them (1,000 rows of 1,000 entries at the end of 100,000 of 13, a product of 8 columns: 364 us by the warps of
+// the rows' own chunks, now 85).
+template <int P, class Span, class Entries, class Quad, class Wide, class LongRow>
+__device__ __forceinline__ void for_rows(std::int64_t n, int chunk, Span&& span, Entries&& entries, Quad&& quad,
+                                         Wide&& wide, LongRow&& long_row) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int group_rows = chunk / kRowWarps, group_lanes = kRowThreads / chunk;
+  const std::int64_t step = gridDim.x * static_cast<std::int64_t>(chunk);
+  const auto group = [&](std::int64_t base, int w) {
+    return base + (w * static_cast<std::int64_t>(gridDim.x) + blockIdx.x) * group_rows;
+  };
+  bool some = false;
+  for (std::int64_t base = 0; base < n; base += step) {
+    const std::int64_t row0 = base + blockIdx.x * static_cast<std::int64_t>(chunk);
+    const std::int64_t end = row0 + chunk < n ? row0 + chunk : n, i = row0 + (threadIdx.x >> 2);
+    const std::int64_t k = group(base, warp) + lane / group_lanes;
+    // (all row pointers are read at once, before the chunk's kind is known)
+    const std::int64_t there = k < n ? entries(k, k + 1) : 0;
+    const auto mine = span(i, end);
+    if (row0 < n) {
+      if (entries(row0, end) > most_entries<P>(chunk) * (end - row0)) wide(row0, end);
+      else if (__any_sync(0xffffffffu, i < end)) quad(i, mine);
+    }
+    some |= there > kLongRow;
+  }
+  if (!__syncthreads_or(some)) return;
+  __shared__ unsigned mask[kRowWarps];
+  for (std::int64_t base = 0; base < n; base += step) {
+    const std::int64_t k = group(base, warp) + lane / group_lanes;
+    const unsigned mine = __ballot_sync(0xffffffffu, lane % group_lanes == 0 && k < n && entries(k, k + 1) > kLongRow);
+    if (lane == 0) mask[warp] = mine;
+    __syncthreads();
+    int turn = 0;
+    for (int w = 0; w < kRowWarps; ++w)
+      for (unsigned m = mask[w]; m; m &= m - 1)
+        if (turn++ % kRowWarps == warp) long_row(group(base, w) + (__ffs(m) - 1) / group_lanes);
+    __syncthreads();  // the masks are written again
   }
 }
 
-template <int P>
-__global__ void __launch_bounds__(256, 3) k_spmm(std::int64_t n, const std::int64_t* rp, const std::int32_t* ci,
-                                                 const double* v, const double* x, std::int64_t ldx, double* y,
-                                                 std::int64_t ldy, int p, double alpha, double beta) {
-  constexpr int K = P >= 4 ? P / 4 : 1;
-  const int lane = threadIdx.x & 31, c0 = quad_col<P>();
-  const std::int64_t warp = (blockIdx.x * static_cast<std::int64_t>(blockDim.x) + threadIdx.x) >> 5;
-  const std::int64_t nwarps = (static_cast<std::int64_t>(gridDim.x) * blockDim.x) >> 5;
+struct SpmmArgs {
+  std::int64_t n;
+  const std::int64_t* rp;
+  const std::int32_t* ci;
+  const double* v;
+  const double* x;
+  std::int64_t ldx;
+  double* y;
+  std::int64_t ldy;
+  int p;
+  double alpha, beta;
+};
+
+// Row i of y = alpha M x + beta y by G lanes; [q0, q1): its entries. All lanes of a warp come here; the rows of
+// those without `store` are not written.
+template <int P, int G, int kAhead>
+__device__ __forceinline__ void spmm_row(const SpmmArgs& g, std::int64_t i, std::int64_t q0, std::int64_t q1,
+                                         bool store) {
   std::int64_t off[P];  // columns beyond p repeat column 0: read, never stored
 #pragma unroll
-  for (int c = 0; c < P; ++c) off[c] = c < p ? c * ldx : 0;
-  for (std::int64_t row0 = 8 * warp; row0 < n; row0 += 8 * nwarps) {
-    const std::int64_t i = row0 + (lane >> 2);
-    double acc[P];
+  for (int c = 0; c < P; ++c) off[c] = c < g.p ? c * g.ldx : 0;
+  double acc[P];
 #pragma unroll
-    for (int c = 0; c < P; ++c) acc[c] = 0.0;
-    auto add = [&](double a, std::int64_t j, double (&t)[P]) {
-      const double* xj = x + j;
+  for (int c = 0; c < P; ++c) acc[c] = 0.0;
+  group_entries<G, kAhead, (P < 8)>(q0, q1, g.ci, g.v, [&](double a, std::int64_t j) {
+    const double* xj = g.x + j;
 #pragma unroll
-      for (int c = 0; c < P; ++c) t[c] = fma(a, xj[off[c]], t[c]);
-    };
-    quad_entries(rp, ci, v, i, i < n, [&](double a, std::int64_t j) { add(a, j, acc); });
-    long_rows(rp, row0, n, [&](std::int64_t row, int owner) {
-      double t[P];
+    for (int c = 0; c < P; ++c) acc[c] = fma(a, xj[off[c]], acc[c]);
+  });
+  const GroupCols<P, G> cols;
+  cols.sum(acc);
 #pragma unroll
-      for (int c = 0; c < P; ++c) t[c] = 0.0;
-      for (std::int64_t q = rp[row] + lane; q < rp[row + 1]; q += 32) add(v[q], ci[q], t);
-#pragma unroll
-      for (int c = 0; c < P; ++c) {
-        const double w = warp_sum(t[c]);
-        if (lane == 4 * owner) acc[c] = w;
-      }
-    });
-    quad_scatter(acc);
-#pragma unroll
-    for (int u = 0; u < K; ++u) {
-      const int c = c0 + u;
-      if (c < p && i < n && (P >= 4 || (lane & (P == 2 ? 1 : 3)) == 0))
-        y[i + c * ldy] = alpha * acc[u] + (beta == 0.0 ? 0.0 : beta * y[i + c * ldy]);
-    }
+  for (int u = 0; u < cols.kCols; ++u) {
+    const int c = cols.first + u;
+    if (c < g.p && store && cols.writer)
+      g.y[i + c * g.ldy] = g.alpha * acc[u] + (g.beta == 0.0 ? 0.0 : g.beta * g.y[i + c * g.ldy]);
   }
+}
+
+// entries that a lane of sixteen or more reads ahead: the loads in flight are these times the columns
+template <int P>
+constexpr int kRowAhead = P >= 4 ? 2 : 4;
+
+template <int P>
+__device__ __noinline__ void spmm_long_row(const SpmmArgs& g, std::int64_t i) {
+  spmm_row<P, 32, kRowAhead<P>>(g, i, g.rp[i], g.rp[i + 1], true);
+}
+
+// the entries of row i < end that its lanes sum: none of a long row
+struct SpmmSpan {
+  std::int64_t q0 = 0, q1 = 0;
+  bool mine = false;
+  __device__ __forceinline__ SpmmSpan(const SpmmArgs& g, std::int64_t i, std::int64_t end) {
+    if (i >= end) return;
+    q0 = g.rp[i];
+    q1 = g.rp[i + 1];
+    mine = q1 - q0 <= kLongRow;
+    if (!mine) q1 = q0;
+  }
+};
+
+template <int P>
+__device__ __noinline__ void spmm_wide_rows(const SpmmArgs& g, std::int64_t row0, std::int64_t end) {
+  for (std::int64_t i = row0 + threadIdx.x / 16; row0 < end; row0 += kRowThreads / 16, i += kRowThreads / 16) {
+    const SpmmSpan e(g, i, end);
+    spmm_row<P, 16, kRowAhead<P>>(g, i, e.q0, e.q1, e.mine);
+  }
+}
+
+template <int P>
+__global__ void __launch_bounds__(kRowThreads, P == 1 ? 5 : (P == 2 ? 4 : 3))
+    k_spmm(const __grid_constant__ SpmmArgs g, int chunk) {
+  for_rows<P>(g.n, chunk, [&](std::int64_t i, std::int64_t end) { return SpmmSpan(g, i, end); },
+              [&](std::int64_t a, std::int64_t b) { return g.rp[b] - g.rp[a]; },
+              [&](std::int64_t i, const SpmmSpan& e) { spmm_row<P, 4, 4>(g, i, e.q0, e.q1, e.mine); },
+              [&](std::int64_t row0, std::int64_t end) { spmm_wide_rows<P>(g, row0, end); },
+              [&](std::int64_t i) { spmm_long_row<P>(g, i); });
 }
 
 // Partial Gram sums: CTA b covers rows [b*chunk, (b+1)*chunk); warp w handles columns i = w, w+8,..
@@ -268,107 +373,166 @@ __global__ void k_fill_normal(std::int64_t n, int p, double* y, std::int64_t ldy
   }
 }
 
-// Shifted residual of a shift-invert solve, four lanes per row and all P columns at once:
+// Shifted residual of a shift-invert solve, all P columns at once:
 //   r(i, c) = (B w_c)(i) - (A y_c)(i),  w = x + sigma y  (B = null: B = I),
 //   s(i, c) = (|B| |w_c|)(i) + (|A| |y_c|)(i),
 // and the componentwise backward error omega_c = max_i |r(i, c)| / s(i, c) with 0/0 = 0, r/0 = inf and
 // inf for a row whose r or s is not finite (the contract of hsolve's shifted_residual,
 // include/hsolve/sparse.hpp:157-174). omega must hold zeros at launch; the maximum is taken by an
 // integer atomic max on the bit patterns of non-negative doubles (order independent).
-template <int P>
-__global__ void __launch_bounds__(256, 3) k_shifted_residual(std::int64_t n, const std::int64_t* arp,
-                                                             const std::int32_t* aci, const double* av,
-                                                             const std::int64_t* brp, const std::int32_t* bci,
-                                                             const double* bv, double sigma, const double* x,
-                                                             std::int64_t ldx, const double* y, std::int64_t ldy,
-                                                             double* r, std::int64_t ldr, int p,
-                                                             unsigned long long* omega) {
-  constexpr int K = P >= 4 ? P / 4 : 1;
-  const int lane = threadIdx.x & 31, c0 = quad_col<P>();
-  const std::int64_t warp = (blockIdx.x * static_cast<std::int64_t>(blockDim.x) + threadIdx.x) >> 5;
-  const std::int64_t nwarps = (static_cast<std::int64_t>(gridDim.x) * blockDim.x) >> 5;
-  const auto xoff = [&](int c) { return c < p ? c * ldx : 0; };  // columns beyond p repeat column 0
+struct ResidualArgs {
+  std::int64_t n;
+  const std::int64_t* arp;
+  const std::int32_t* aci;
+  const double* av;
+  const std::int64_t* brp;
+  const std::int32_t* bci;
+  const double* bv;
+  double sigma;
+  const double* x;
+  std::int64_t ldx;
+  const double* y;
+  std::int64_t ldy;
+  double* r;
+  std::int64_t ldr;
+  int p;
+};
+
+// Row i by G lanes ([a0, a1), [b0, b1): its entries of A and B): r stored and om raised to the row's backward
+// errors where `store` (the lanes' columns, see GroupCols).
+template <int P, int G, int kAhead, class Om>
+__device__ __forceinline__ void residual_row(const ResidualArgs& g, std::int64_t i, std::int64_t a0, std::int64_t a1,
+                                             std::int64_t b0, std::int64_t b1, bool store, Om&& om) {
+  const auto xoff = [&](int c) { return c < g.p ? c * g.ldx : 0; };  // columns beyond p repeat column 0
   std::int64_t yoff[P];
 #pragma unroll
-  for (int c = 0; c < P; ++c) yoff[c] = c < p ? c * ldy : 0;
-  double om[K];
+  for (int c = 0; c < P; ++c) yoff[c] = c < g.p ? c * g.ldy : 0;
+  double ra[P], sa[P];
 #pragma unroll
-  for (int u = 0; u < K; ++u) om[u] = 0.0;
-  for (std::int64_t row0 = 8 * warp; row0 < n; row0 += 8 * nwarps) {
-    const std::int64_t i = row0 + (lane >> 2);
-    const bool in = i < n;
-    double ra[P], sa[P];
+  for (int c = 0; c < P; ++c) { ra[c] = 0.0; sa[c] = 0.0; }
+  group_entries<G, kAhead, (P < 8)>(a0, a1, g.aci, g.av, [&](double a, std::int64_t j) {
+    const double* yj = g.y + j;
 #pragma unroll
-    for (int c = 0; c < P; ++c) { ra[c] = 0.0; sa[c] = 0.0; }
-    auto add_a = [&](double a, std::int64_t j, double (&rr)[P], double (&ss)[P]) {
-      const double* yj = y + j;
-#pragma unroll
-      for (int c = 0; c < P; ++c) {
-        const double t = yj[yoff[c]];
-        rr[c] = fma(-a, t, rr[c]);
-        ss[c] = fma(fabs(a), fabs(t), ss[c]);
-      }
-    };
-    auto add_b = [&](double b, std::int64_t j, double (&rr)[P], double (&ss)[P]) {
+    for (int c = 0; c < P; ++c) {
+      const double t = yj[yoff[c]];
+      ra[c] = fma(-a, t, ra[c]);
+      sa[c] = fma(fabs(a), fabs(t), sa[c]);
+    }
+  });
+  if (g.brp)
+    group_entries<G, kAhead, (P < 8)>(b0, b1, g.bci, g.bv, [&](double b, std::int64_t j) {
 #pragma unroll
       for (int c = 0; c < P; ++c) {
-        const double w = fma(sigma, y[j + yoff[c]], x[j + xoff(c)]);
-        rr[c] = fma(b, w, rr[c]);
-        ss[c] = fma(fabs(b), fabs(w), ss[c]);
+        const double w = fma(g.sigma, g.y[j + yoff[c]], g.x[j + xoff(c)]);
+        ra[c] = fma(b, w, ra[c]);
+        sa[c] = fma(fabs(b), fabs(w), sa[c]);
       }
-    };
-    quad_entries(arp, aci, av, i, in, [&](double a, std::int64_t j) { add_a(a, j, ra, sa); });
-    if (brp) quad_entries(brp, bci, bv, i, in, [&](double b, std::int64_t j) { add_b(b, j, ra, sa); });
-    auto by_warp = [&](const std::int64_t* rp, const std::int32_t* ci, const double* v, auto&& add) {
-      long_rows(rp, row0, n, [&](std::int64_t row, int owner) {
-        double rr[P], ss[P];
+    });
+  const GroupCols<P, G> cols;
+  cols.sum(ra);
+  cols.sum(sa);
 #pragma unroll
-        for (int c = 0; c < P; ++c) { rr[c] = 0.0; ss[c] = 0.0; }
-        for (std::int64_t q = rp[row] + lane; q < rp[row + 1]; q += 32) add(v[q], ci[q], rr, ss);
-#pragma unroll
-        for (int c = 0; c < P; ++c) {
-          const double tr = warp_sum(rr[c]), ts = warp_sum(ss[c]);
-          if (lane == 4 * owner) { ra[c] += tr; sa[c] += ts; }
-        }
-      });
-    };
-    by_warp(arp, aci, av, add_a);
-    if (brp) by_warp(brp, bci, bv, add_b);
-    quad_scatter(ra);
-    quad_scatter(sa);
-#pragma unroll
-    for (int u = 0; u < K; ++u) {
-      const int c = c0 + u;
-      if (c >= p || !in) continue;
-      double rs = ra[u], ss = sa[u];
-      if (!brp) {
-        const double w = fma(sigma, y[i + c * ldy], x[i + c * ldx]);
-        rs += w;
-        ss += fabs(w);
-      }
-      if (r && (P >= 4 || (lane & (P == 2 ? 1 : 3)) == 0)) r[i + c * ldr] = rs;
-      const double ar = fabs(rs);
-      double w;
-      if (!isfinite(rs) || !isfinite(ss)) w = CUDART_INF;
-      else if (ss > 0.0) w = ar / ss;
-      else w = ar > 0.0 ? CUDART_INF : 0.0;
-      om[u] = fmax(om[u], w);
+  for (int u = 0; u < cols.kCols; ++u) {
+    const int c = cols.first + u;
+    if (c >= g.p || !store) continue;
+    double rs = ra[u], ss = sa[u];
+    if (!g.brp) {
+      const double w = fma(g.sigma, g.y[i + c * g.ldy], g.x[i + c * g.ldx]);
+      rs += w;
+      ss += fabs(w);
+    }
+    if (g.r && cols.writer) g.r[i + c * g.ldr] = rs;
+    const double ar = fabs(rs);
+    double w;
+    if (!isfinite(rs) || !isfinite(ss)) w = CUDART_INF;
+    else if (ss > 0.0) w = ar / ss;
+    else w = ar > 0.0 ? CUDART_INF : 0.0;
+    om(u, w);
+  }
+}
+
+// (om: the warp's own column maxima in shared memory)
+template <int P>
+__device__ __noinline__ void residual_long_row(const ResidualArgs& g, std::int64_t i, double* om) {
+  const GroupCols<P, 32> cols;
+  residual_row<P, 32, kRowAhead<P>>(g, i, g.arp[i], g.arp[i + 1], g.brp ? g.brp[i] : 0, g.brp ? g.brp[i + 1] : 0, true,
+                                    [&](int u, double w) {
+                                      if (cols.writer) om[cols.first + u] = fmax(om[cols.first + u], w);
+                                    });
+  __syncwarp();
+}
+
+// the entries of row i < end that its lanes sum: none of a long row
+struct ResidualSpan {
+  std::int64_t a0 = 0, a1 = 0, b0 = 0, b1 = 0;
+  bool mine = false;
+  __device__ __forceinline__ ResidualSpan(const ResidualArgs& g, std::int64_t i, std::int64_t end) {
+    if (i >= end) return;
+    a0 = g.arp[i];
+    a1 = g.arp[i + 1];
+    if (g.brp) {
+      b0 = g.brp[i];
+      b1 = g.brp[i + 1];
+    }
+    mine = a1 - a0 <= kLongRow && b1 - b0 <= kLongRow;
+    if (!mine) {
+      a1 = a0;
+      b1 = b0;
     }
   }
+};
+
+// the lanes' column maxima to the warp's (part)
+template <int P, int G>
+__device__ __forceinline__ void keep_maxima(const double (&om)[GroupCols<P, G>::kCols], double* part) {
+  const GroupCols<P, G> cols;
+#pragma unroll
+  for (int u = 0; u < cols.kCols; ++u) {
+    double w = om[u];
+#pragma unroll
+    for (int o = G; o < 32; o <<= 1) w = fmax(w, __shfl_xor_sync(0xffffffffu, w, o));
+    if ((threadIdx.x & 31) < G && cols.writer) part[cols.first + u] = fmax(part[cols.first + u], w);
+  }
+  __syncwarp();
+}
+template <int P>
+__device__ __noinline__ void residual_wide_rows(const ResidualArgs& g, std::int64_t row0, std::int64_t end,
+                                                double* part) {
+  double om[GroupCols<P, 16>::kCols] = {};
+  for (std::int64_t i = row0 + threadIdx.x / 16; row0 < end; row0 += kRowThreads / 16, i += kRowThreads / 16) {
+    const ResidualSpan e(g, i, end);
+    residual_row<P, 16, kRowAhead<P>>(g, i, e.a0, e.a1, e.b0, e.b1, e.mine,
+                                      [&](int u, double w) { om[u] = fmax(om[u], w); });
+  }
+  keep_maxima<P, 16>(om, part);
+}
+
+template <int P>
+__global__ void __launch_bounds__(kRowThreads, P == 1 ? 4 : 3)
+    k_shifted_residual(const __grid_constant__ ResidualArgs g, int chunk, unsigned long long* omega) {
+  __shared__ double part[kRowWarps][P];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane < P) part[warp][lane] = 0.0;
+  __syncwarp();
+  double om[GroupCols<P, 4>::kCols] = {};
+  const auto entries = [&](std::int64_t a, std::int64_t b) {
+    const std::int64_t in_a = g.arp[b] - g.arp[a], in_b = g.brp ? g.brp[b] - g.brp[a] : 0;
+    return in_a > in_b ? in_a : in_b;
+  };
+  for_rows<P>(g.n, chunk, [&](std::int64_t i, std::int64_t end) { return ResidualSpan(g, i, end); }, entries,
+           [&](std::int64_t i, const ResidualSpan& e) {
+             residual_row<P, 4, 4>(g, i, e.a0, e.a1, e.b0, e.b1, e.mine,
+                                   [&](int u, double w) { om[u] = fmax(om[u], w); });
+           },
+           [&](std::int64_t row0, std::int64_t end) { residual_wide_rows<P>(g, row0, end, part[warp]); },
+           [&](std::int64_t i) { residual_long_row<P>(g, i, part[warp]); });
+  keep_maxima<P, 4>(om, part[warp]);
   if (omega) {
     // one atomic per column and CTA
-    __shared__ double part[8][P];
-#pragma unroll
-    for (int u = 0; u < K; ++u) {
-      double w = om[u];
-#pragma unroll
-      for (int o = 4; o < 32; o <<= 1) w = fmax(w, __shfl_xor_sync(0xffffffffu, w, o));
-      if (lane < 4) part[threadIdx.x >> 5][c0 + u] = w;
-    }
     __syncthreads();
-    if (threadIdx.x < P && static_cast<int>(threadIdx.x) < p) {
+    if (threadIdx.x < P && static_cast<int>(threadIdx.x) < g.p) {
       double w = 0.0;
-      for (int q = 0; q < 8; ++q) w = fmax(w, part[q][threadIdx.x]);
+      for (int q = 0; q < kRowWarps; ++q) w = fmax(w, part[q][threadIdx.x]);
       if (w > 0.0) atomic_max_nonneg(&omega[threadIdx.x], w);
     }
   }
@@ -440,21 +604,24 @@ int grid_for(std::int64_t work, int threads) {
   return static_cast<int>(b < 1 ? 1 : (b > 148 * 32 ? 148 * 32 : b));
 }
 
+// rows of a CTA's chunk, and the CTAs: chunks are short while the matrix has too few rows for three CTAs an SM
+int row_chunk(std::int64_t n) { return n <= kSmallRows ? kSmallChunk : kChunk; }
+int row_grid(std::int64_t n) { return grid_for(n * (kRowThreads / row_chunk(n)), kRowThreads); }
+
 }  // namespace
 
 void spmm(const CsrDev& M, const double* x, std::int64_t ldx, double* y, std::int64_t ldy, int p, double alpha,
           double beta, cudaStream_t s) {
   if (p <= 0 || M.n == 0) return;
-  const int threads = 256;
-  const int blocks = grid_for(M.n * 4, threads);
+  const int blocks = row_grid(M.n), chunk = row_chunk(M.n);
   for (int c0 = 0; c0 < p; c0 += 8) {
     const int pc = p - c0 < 8 ? p - c0 : 8;
     const double* xc = x + c0 * ldx;
-    double* yc = y + c0 * ldy;
-    if (pc == 1) { note_launches(1); k_spmm<1><<<blocks, threads, 0, s>>>(M.n, M.rp, M.ci, M.v, xc, ldx, yc, ldy, pc, alpha, beta); }
-    else if (pc <= 2) { note_launches(1); k_spmm<2><<<blocks, threads, 0, s>>>(M.n, M.rp, M.ci, M.v, xc, ldx, yc, ldy, pc, alpha, beta); }
-    else if (pc <= 4) { note_launches(1); k_spmm<4><<<blocks, threads, 0, s>>>(M.n, M.rp, M.ci, M.v, xc, ldx, yc, ldy, pc, alpha, beta); }
-    else { note_launches(1); k_spmm<8><<<blocks, threads, 0, s>>>(M.n, M.rp, M.ci, M.v, xc, ldx, yc, ldy, pc, alpha, beta); }
+    const SpmmArgs g{M.n, M.rp, M.ci, M.v, xc, ldx, y + c0 * ldy, ldy, pc, alpha, beta};
+    if (pc == 1) { note_launches(1); k_spmm<1><<<blocks, kRowThreads, 0, s>>>(g, chunk); }
+    else if (pc <= 2) { note_launches(1); k_spmm<2><<<blocks, kRowThreads, 0, s>>>(g, chunk); }
+    else if (pc <= 4) { note_launches(1); k_spmm<4><<<blocks, kRowThreads, 0, s>>>(g, chunk); }
+    else { note_launches(1); k_spmm<8><<<blocks, kRowThreads, 0, s>>>(g, chunk); }
   }
 }
 
@@ -574,8 +741,7 @@ void shifted_residual(const CsrDev& A, const CsrDev* B, double sigma, const doub
                       const double* y, std::int64_t ldy, double* r, std::int64_t ldr, int p, double* omega,
                       cudaStream_t s) {
   if (p <= 0 || A.n == 0) return;
-  const int threads = 256;
-  const int blocks = grid_for(A.n * 4, threads);
+  const int blocks = row_grid(A.n), chunk = row_chunk(A.n);
   if (omega) cuda_check(cudaMemsetAsync(omega, 0, static_cast<std::size_t>(p) * sizeof(double), s), "memset omega");
   for (int c0 = 0; c0 < p; c0 += 8) {
     const int pc = p - c0 < 8 ? p - c0 : 8;
@@ -583,18 +749,17 @@ void shifted_residual(const CsrDev& A, const CsrDev* B, double sigma, const doub
     const double* yc = y + c0 * ldy;
     double* rc = r ? r + c0 * ldr : nullptr;
     unsigned long long* oc = omega ? reinterpret_cast<unsigned long long*>(omega + c0) : nullptr;
-    const std::int64_t* brp = B ? B->rp : nullptr;
-    const std::int32_t* bci = B ? B->ci : nullptr;
-    const double* bvv = B ? B->v : nullptr;
+    const ResidualArgs g{A.n, A.rp, A.ci, A.v, B ? B->rp : nullptr, B ? B->ci : nullptr, B ? B->v : nullptr, sigma,
+                         xc, ldx, yc, ldy, rc, ldr, pc};
     note_launches(1);
     if (pc == 1)
-      k_shifted_residual<1><<<blocks, threads, 0, s>>>(A.n, A.rp, A.ci, A.v, brp, bci, bvv, sigma, xc, ldx, yc, ldy, rc, ldr, pc, oc);
+      k_shifted_residual<1><<<blocks, kRowThreads, 0, s>>>(g, chunk, oc);
     else if (pc <= 2)
-      k_shifted_residual<2><<<blocks, threads, 0, s>>>(A.n, A.rp, A.ci, A.v, brp, bci, bvv, sigma, xc, ldx, yc, ldy, rc, ldr, pc, oc);
+      k_shifted_residual<2><<<blocks, kRowThreads, 0, s>>>(g, chunk, oc);
     else if (pc <= 4)
-      k_shifted_residual<4><<<blocks, threads, 0, s>>>(A.n, A.rp, A.ci, A.v, brp, bci, bvv, sigma, xc, ldx, yc, ldy, rc, ldr, pc, oc);
+      k_shifted_residual<4><<<blocks, kRowThreads, 0, s>>>(g, chunk, oc);
     else
-      k_shifted_residual<8><<<blocks, threads, 0, s>>>(A.n, A.rp, A.ci, A.v, brp, bci, bvv, sigma, xc, ldx, yc, ldy, rc, ldr, pc, oc);
+      k_shifted_residual<8><<<blocks, kRowThreads, 0, s>>>(g, chunk, oc);
   }
 }
 
