@@ -971,6 +971,10 @@ bool GpuFactor::capture(const std::function<void()>& direct, cudaGraphExec_t* ex
   return ok;
 }
 
+// Solves captured at once by an object, one per number of right-hand sides (and per place of the work arrays,
+// which move when a wider solve comes); the one that was used longest ago goes first.
+constexpr std::size_t kSolveGraphs = 64;
+
 void GpuFactor::run_solve(double* b, std::int64_t ld, double* xwork, double* vec, int nr, bool graph) {
   pinned_->rhs = SolveRhs{b, ld};
   auto direct = [&] {
@@ -984,11 +988,12 @@ void GpuFactor::run_solve(double* b, std::int64_t ld, double* xwork, double* vec
     cuda_check(cudaMemcpyAsync(&pinned_->err, d_err_.p, sizeof(int), cudaMemcpyDeviceToHost, s), "solve status");
   };
   if (!graph || !graphs_ok_) return direct();
-  for (const SweepGraph& g : graphs_)
-    if (g.xwork == xwork && g.vec == vec && g.nr == nr) {
-      note_launches(g.launches);
+  for (auto g = graphs_.begin(); g != graphs_.end(); ++g)
+    if (g->xwork == xwork && g->vec == vec && g->nr == nr) {
+      std::rotate(g, g + 1, graphs_.end());  // the last used comes last
+      note_launches(graphs_.back().launches);
       ++solve_replays_;
-      cuda_check(cudaGraphLaunch(g.exec, stream_), "solve (graph)");
+      cuda_check(cudaGraphLaunch(graphs_.back().exec, stream_), "solve (graph)");
       return;
     }
   // capture the sequence once; where capturing is refused (e.g. a cooperative launch), launch
@@ -998,6 +1003,10 @@ void GpuFactor::run_solve(double* b, std::int64_t ld, double* xwork, double* vec
   if (!capture(direct, &exec, &captured)) {
     graphs_ok_ = false;
     return direct();
+  }
+  if (graphs_.size() == kSolveGraphs) {  // (its last solve is complete: every solve waits for its own)
+    cudaGraphExecDestroy(graphs_.front().exec);
+    graphs_.erase(graphs_.begin());
   }
   graphs_.push_back(SweepGraph{xwork, vec, nr, captured, exec});
   note_launches(captured);

@@ -11,6 +11,7 @@ from helpers import laplacian_1d, laplacian_2d
 pytestmark = pytest.mark.gpu
 
 USES = 8  # a form's first captured use
+SOLVE_GRAPHS = 64  # most captured solves of an object
 LARGEST = 65536  # largest order whose factorizations are captured
 
 
@@ -71,6 +72,24 @@ def test_orders_around_the_largest_captured(n):
         c = f.count(1.0, 0.0)
         assert (c.neg, c.zero, c.pos) == (0, 0, n)
     assert f.graph_stats()["factor_replays"] == (2 if n <= LARGEST else 0)
+
+
+def test_captured_solves_are_bounded():
+    from hsolve_b200 import Factorization
+
+    a = laplacian_2d(9, 7)
+    f = Factorization(device=0)
+    f.analyze(a, None, 1.0, 0.0)
+    assert f.factorize(1.0, 0.0)
+    b = np.random.default_rng(2).standard_normal((a.shape[0], 150))
+    want = np.linalg.solve(a.toarray(), b)
+    for p in [*range(1, 151), 150, 3, 149, 1]:  # each width moves the work arrays up to 150
+        x = f.solve(b[:, :p])
+        # a symmetric positive definite matrix with a condition below 100
+        assert np.abs(x - want[:, :p]).max() <= 100 * a.shape[0] * np.finfo(float).eps * np.abs(want).max()
+        assert f.graph_stats()["solve_graphs"] <= SOLVE_GRAPHS
+    assert f.graph_stats()["solve_graphs"] == SOLVE_GRAPHS
+    assert f.graph_stats()["solve_replays"] == 154
 
 
 def test_two_threads_replay_their_own_objects():
