@@ -96,6 +96,25 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// Asynchronous copy of one factor element (sizeof(R) bytes) from global to shared memory;
+// valid == false fills the destination with zero.
+template <class R>
+__device__ __forceinline__ void cp_async_elem(R* dst, const R* src, bool valid) {
+  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+  if constexpr (sizeof(R) == 8) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(valid ? 8 : 0) : "memory");
+  } else {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(valid ? 4 : 0) : "memory");
+  }
+}
+
+// D = A B + D on the FP64 tensor cores, A 8 x 4, B 4 x 8: a lane holds A(lane / 4, lane % 4), B(lane % 4, lane / 4)
+// and columns 2 (lane % 4), + 1 of row lane / 4 of D.
+__device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(d0), "+d"(d1) : "d"(a), "d"(b));
+}
+
 #endif  // __CUDACC__
 
 }  // namespace hsg

@@ -2,7 +2,7 @@
 //
 // What replaces MUMPS JOB=2 (hsolve src/factor/mumps_factorization.cpp:300-356; the arithmetic of
 // MUMPS dfac_front_LDLT_type1.F / dfac_front_aux.F / dfac_asm.F): symmetric equilibration of
-// K = alpha A + beta B, scatter of K into the fronts' panels, extend-add of children's contribution
+// K = alpha A + beta B, scatter of K into the fronts' panels, assembly of children's contribution
 // blocks, and the partial factorization of every front with 1x1 / 2x2 threshold pivots restricted
 // to its fully-summed columns. Inertia (neg / zero / pos) is counted from D as pivots are accepted.
 //
@@ -41,19 +41,7 @@ __device__ __forceinline__ double pivot_det(double a, double b, double c) {
 __device__ __forceinline__ double2 load_pair(const double* p) { return *reinterpret_cast<const double2*>(p); }
 __device__ __forceinline__ float2 load_pair(const float* p) { return *reinterpret_cast<const float2*>(p); }
 
-// Asynchronous copy of one factor element (sizeof(R) bytes) from global to shared memory;
-// valid == false fills the destination with zero.
-template <class R>
-__device__ __forceinline__ void cp_async_elem(R* dst, const R* src, bool valid) {
-  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-  if constexpr (sizeof(R) == 8) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(valid ? 8 : 0) : "memory");
-  } else {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(valid ? 4 : 0) : "memory");
-  }
-}
-
-// the same to a shared-memory address, of `size` bytes (sizeof(R), or 0: filled with zero)
+// cp_async_elem to a shared-memory address, of `size` bytes (sizeof(R), or 0: filled with zero)
 template <class R>
 __device__ __forceinline__ void cp_async_sized(unsigned dst, const R* src, int size) {
   if constexpr (sizeof(R) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(size) : "memory");
@@ -66,12 +54,6 @@ __global__ void k_fill(double* x, std::int64_t n, double v) {
   for (std::int64_t i = blockIdx.x * static_cast<std::int64_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<std::int64_t>(gridDim.x) * blockDim.x)
     x[i] = v;
-}
-
-__global__ void k_zero_u64(unsigned long long* x, std::int64_t n) {
-  for (std::int64_t i = blockIdx.x * static_cast<std::int64_t>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<std::int64_t>(gridDim.x) * blockDim.x)
-    x[i] = 0ull;
 }
 
 // The kernels that form K = alpha A + beta B read (alpha, beta) = ab[0..1] from device memory, so that a
@@ -387,11 +369,6 @@ __device__ void dense_bk_step(R* F, int ld, int m, int nfs, bool root, double u,
     break;
   }
   __syncthreads();
-}
-
-__device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(d0), "+d"(d1) : "d"(a), "d"(b));
 }
 
 constexpr double kRcpMin = 1e-280, kRcpMax = 1e280;  // |d| whose reciprocal is away from the ends of the range
@@ -1851,13 +1828,6 @@ void launch_fill(double* x, std::int64_t n, double v, cudaStream_t s) {
   const int blocks = static_cast<int>(std::min<std::int64_t>((n + 255) / 256, 148 * 16));
   note_launches(1);
   k_fill<<<blocks, 256, 0, s>>>(x, n, v);
-}
-
-void launch_zero_u64(unsigned long long* x, std::int64_t n, cudaStream_t s) {
-  if (n <= 0) return;
-  const int blocks = static_cast<int>(std::min<std::int64_t>((n + 255) / 256, 148 * 16));
-  note_launches(1);
-  k_zero_u64<<<blocks, 256, 0, s>>>(x, n);
 }
 
 void launch_scale_rowmax(std::int64_t nnz, const std::int32_t* row, const std::int32_t* col, const double* a,

@@ -30,7 +30,6 @@ constexpr int kRowStage = kNB * kNB + 4 * kNB;   // panel row step: the block's 
 constexpr int kRowChunk = (kAppDynDoubles - kRowStage) / kNB;  // rows staged at once by the panel row step
 constexpr int kAppThreads = 256;
 constexpr int kCoopMinFront = 192;     // levels whose largest panel front is at least this use the cooperative kernel
-constexpr int kColsPerThread = kTile * kTile / kAppThreads;  // 16
 constexpr int kAssembleCols = 8;       // columns per assembly CTA (a warp each)
 // per-front scratch of the panel kernels (doubles): control block, two sets (alternate panels) of
 // block, original block, labels, pivot types and column maxima, backup of the panel's rows, W = L D
@@ -42,7 +41,6 @@ inline std::int64_t app_scratch_doubles(int m, int k) {
 }
 
 void launch_fill(double* x, std::int64_t n, double v, cudaStream_t s);
-void launch_zero_u64(unsigned long long* x, std::int64_t n, cudaStream_t s);
 void launch_scale_rowmax(std::int64_t nnz, const std::int32_t* row, const std::int32_t* col, const double* a,
                          const double* b, const double* ab, const double* d, unsigned long long* r,
                          cudaStream_t s);

@@ -634,8 +634,6 @@ std::shared_ptr<FrontPlan> GpuFactor::make_plan() {
   P.items.upload(items, stream_);
   P.rmap.upload(S.rmap, stream_);
   P.rows.upload(rows, stream_);
-  P.child_ptr.upload(S.child_ptr, stream_);
-  P.children.upload(S.children, stream_);
   P.iperm.upload(S.iperm, stream_);
   P.dest.upload(S.dest, stream_);
   P.tasks.upload(tasks, stream_);

@@ -120,8 +120,8 @@ struct FrontPlan {
   DevBuf<std::int32_t> row, col;   // the union pattern's entries (row, column)
   DevBuf<std::int64_t> dest;       // their positions in the factor storage
   DevBuf<SnDev> sn;
-  DevBuf<std::int32_t> lists, rmap, rows, child_ptr, children, iperm;
-  DevBuf<int2> items;              // extend-add items by child rank
+  DevBuf<std::int32_t> lists, rmap, rows, iperm;
+  DevBuf<int2> items;              // assembly CTAs by level: front, first of its columns
   // inertia-only counts: fronts with arena offsets, entries by level and their arena destinations
   DevBuf<SnDev> sn_cnt;
   DevBuf<std::int64_t> ent_idx, dest_cnt;

@@ -89,16 +89,8 @@ __global__ void k_solve_diag_flat(std::int64_t npiv, const std::int64_t* dpos, c
 
 namespace {
 
-__device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
-}
-
 // factor entry to a double in shared memory (zero where not valid): asynchronously for FP64 factors
-__device__ __forceinline__ void stage_entry(double* dst, const double* src, bool valid) {
-  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(valid ? 8 : 0) : "memory");
-}
+__device__ __forceinline__ void stage_entry(double* dst, const double* src, bool valid) { cp_async_elem(dst, src, valid); }
 __device__ __forceinline__ void stage_entry(double* dst, const float* src, bool valid) {
   *dst = valid ? static_cast<double>(*src) : 0.0;
 }
@@ -191,7 +183,7 @@ __global__ void __launch_bounds__(256) k_sb_narrow(const int4* items, const SnDe
       const double a = L[(s0 + t4) * kRowsLd + 8 * warp + g];
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        if (8 * q <= s0 + 3) dmma_8x8x4(acc[q], a, Xs[(8 * q + g) * kXLd + s0 + t4]);
+        if (8 * q <= s0 + 3) dmma_m8n8k4(acc[q][0], acc[q][1], a, Xs[(8 * q + g) * kXLd + s0 + t4]);
     }
     const int i = r0 + 64 * t + 8 * warp + g;
 #pragma unroll
@@ -241,7 +233,7 @@ __global__ void __launch_bounds__(256) k_sb_inverse(const int2* sbl, const SnDev
 #pragma unroll
       for (int u = 0; u < 6; ++u) {
         const int q = 2 * u + h;
-        if (8 * q <= s0 + 3 && 8 * q < o) dmma_8x8x4(acc[u], a, S[(8 * q + g) * kInvLd + s0 + t4]);
+        if (8 * q <= s0 + 3 && 8 * q < o) dmma_m8n8k4(acc[u][0], acc[u][1], a, S[(8 * q + g) * kInvLd + s0 + t4]);
       }
     }
 #pragma unroll
@@ -322,7 +314,7 @@ __global__ void __launch_bounds__(256, 2) k_sb_apply(const int4* tiles, const Sn
       const int nq = min((j0 + s0) / 8 + 1, (bs + 7) / 8);
 #pragma unroll
       for (int q = 0; q < kSB / 8; ++q)
-        if (q < nq) dmma_8x8x4(acc[q], a, Xs[(8 * q + g) * kXLd + s0 + t4]);
+        if (q < nq) dmma_m8n8k4(acc[q][0], acc[q][1], a, Xs[(8 * q + g) * kXLd + s0 + t4]);
     }
     __syncthreads();
   }
