@@ -552,9 +552,9 @@ __device__ __forceinline__ float warp_maxf(float v) {
 
 // One warp: one elimination of threshold Bunch-Kaufman on the panel's diagonal block (order w <= 32,
 // shared memory, ld kNB, all rows candidates), from the state in st: the general step, for the columns
-// where fast_pivots stops. Same acceptance rules as dense_bk_step; column maxima are reduced in
-// single precision (a threshold test needs no more), the argmax for a 2 x 2 partner only when the
-// 1 x 1 test fails, one reciprocal per pivot. The update of a step reads the pivot column(s) into
+// where fast_pivots stops. The acceptance rules of dense_bk_step, up to the column maxima's rounding to
+// single precision (the panel's rows test every pivot again); the argmax for a 2 x 2 partner is taken only
+// where the 1 x 1 test fails; columns are scaled by 1 / d or by the inverse of the 2 x 2 pivot. The update of a step reads the pivot column(s) into
 // registers first, so its column read-modify-writes are independent and pipeline. Not inlined: as a
 // function of its own it is register-allocated apart from the panel kernels' other phases.
 // Warp-synchronous: no block barriers. Ends after a pivot or with st.stop = 1 ([st.j, w) could not be
@@ -1053,8 +1053,8 @@ __device__ void app_control_and_block(AppFront<R>& F, const FactorParams& prm, d
 // columns) and write the backup, and a warp per four columns applies D^-1 through per-column
 // coefficients (no branch on the pivot type), writes L and W = L D back (coalesced) and reduces the
 // column maxima. The phase is a chain of latencies (a rank of the n = 109,744 box's root holds at most
-// 45 rows): with one thread a row (496 dependent-load FMAs, 3.3 us) and the copies after the block it
-// took 7.9 us a panel, now 5.3.
+// 20 rows): with 64 CTAs there, at most 45 rows each, one thread a row (496 dependent-load FMAs, 3.3 us) and
+// the copies after the block took 7.9 us a panel, this form 5.3; with 148 CTAs it is 5.5.
 template <class R>
 __device__ void app_rows(AppFront<R>& F, const StepView& v, int rank, int nr, R* Bs, int* slab, signed char* spv,
                          R* Lm) {
@@ -1349,9 +1349,9 @@ __device__ __forceinline__ bool app_flushes(int m, int p, int w, int q, int lim,
 // W come in chunks of kUpdChunk pivots by cp.async (zero-filled outside the front), column-major with
 // stride kUpdLd = 4 (mod 16): copies of consecutive rows are contiguous and every fragment read of a
 // half-warp hits 32 distinct banks. kUpdStages chunks are in flight across tile boundaries, so the
-// next tile arrives while this one is computed (a 64 x 64 x 128 tile is 4.5 us of FP64 tensor work on
+// next tile arrives while this one is computed (a 64 x 64 x 128 tile is 4.2 us of FP64 tensor work on
 // an SM; staged as a whole, scaled by D and only then multiplied, the update phase of a root panel of
-// the n = 109,744 box took 20.0 us, now 16.1; factorize + 8 solves there 21.4 -> 18.5 ms).
+// the n = 109,744 box took 20.0 us with 64 CTAs, this form 16.1; with 148 CTAs it is 10.4).
 // Warp w (of 8) computes rows 16 (w % 4) .. +16 and columns 32 (w / 4) .. +32
 // of the tile as 2 x 4 blocks of 8 x 8. A thread's fragment element (g, t) is row g = lane / 4,
 // column t = lane % 4 of A; row t, column g of B; row g, columns 2t, 2t + 1 of C.
@@ -1361,8 +1361,8 @@ __device__ __forceinline__ bool app_flushes(int m, int p, int w, int q, int lim,
 //
 // With look-ahead (la: the panel was accepted whole and the next one follows directly), rank 0 updates
 // and factorizes the next panel's diagonal block first (app_next_block): that block is left out here, and
-// rank 0 takes the last tiles of the list, fewer than the others by what its block costs (about 8 us: two
-// tiles of 128 pivots, five of 32).
+// rank 0 takes the last tiles of the list, fewer than the others by what its block costs (about 9.5 us: two
+// tiles of 128 pivots, five of 32; of 224 pivots it is rather one, which gains 0.6 % at n = 291,359).
 struct UpdTile {
   int tile, ti, tj;
 };

@@ -696,10 +696,12 @@ std::size_t GpuFactor::factor_bytes() const {
 }
 
 // The launches of a small factorization are queued from one graph once a form has been used kGraphUses
-// times: 50 to 120 launches at 5.3 us of host time each, 0.6 to 1.1 us in a graph, bound it (a count at
-// n = 737: 492 us, 379 from the graph; a factorization at n = 3,021: 770 and 650). Capturing and
-// instantiating costs 2 to 3 ms once, so that a few factorizations would not win it back, and above
-// kGraphOrder the launches hide behind the kernels (n = 109,744: 12.4 and 12.3 ms).
+// times: 50 to 120 launches at 5.3 us of host time each, 0.6 to 1.1 us in a graph, bound it. Counts launched
+// directly and from the graph: n = 737 470 and 375 us, 3,021 760 and 665, 10,064 1,535 and 1,410, 21,660
+// 2,665 and 2,620, 58,885 5.80 and 5.60 ms; a factorization at n = 109,744 12.4 and 12.3 ms, where the
+// launches hide behind the kernels. A capture costs 0.13 to 0.30 ms in the call that makes it, won back by two
+// or three further uses (n = 21,660: four), and the first of a process 1 to 2.4 ms more: objects of a few
+// factorizations do not pay it.
 constexpr int kGraphUses = 8;
 constexpr std::int64_t kGraphOrder = 65536;
 

@@ -154,7 +154,7 @@ class GpuFactor {
   void analyze_like(const GpuFactor& src);
   void solve(double* b, std::int64_t nrhs, std::int64_t ldb, bool on_device);
   // Doubles of work space that solve_with_scratch needs for nrhs right-hand sides: n x nrhs for the
-  // permuted, scaled right-hand sides and (contribution rows) x min(nrhs, 8) for the update vectors.
+  // permuted, scaled right-hand sides and (contribution rows) x min(nrhs, 16) for the update vectors.
   std::size_t solve_scratch_doubles(std::int64_t nrhs) const;
   // The solve of a device-resident b (column-major, leading dimension ldb) with its work space in
   // the caller's `scratch` (`cap` doubles, on this factorization's device). Allocates no device
@@ -275,8 +275,7 @@ class GpuFactor {
   std::vector<SweepGraph> graphs_;
   long long factor_replays_ = 0, solve_replays_ = 0;
   // captured factorizations by what their launches depend on beside the shift (which they read from
-  // pinned_), once a form has been used often enough to win the capture back; valid until the plan or the
-  // buffers change
+  // pinned_), once a form has been used a few times; valid until the plan or the buffers change
   struct FactorGraph {
     bool detection, count_only, shared;
     const void* panels;
