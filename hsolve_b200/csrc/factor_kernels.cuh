@@ -14,10 +14,11 @@ constexpr int kTile = 64;              // trailing-update tile (rows = cols)
 // Pending pivots whose trailing update is applied at once (blocked step). More of them spread a tile's fixed
 // costs and its pass over C over more products, but lengthen the next panel's own updates, which are on
 // the chain: n = 291,359 (fronts to 5,861) 53.7 ms a factorization with 128, 52.3 with 192, 51.9 with 224;
-// n = 21,660 (fronts to 1,279) 2.61, 2.63, 2.65. With 224 from an order of 1,400 on: 51.8 and 2.61 ms, from
-// 2,048 on 52.2, from 3,000 on 52.2.
+// n = 21,660 (fronts to 1,279) 2.61, 2.63, 2.65. With 224 in no front, from an order of 2,048 on and from
+// 1,400 on (ms): n = 48,750 (fronts to 1,961) 5.22, 5.22, 5.30; 58,885 (1,966) 5.63, 5.63, 5.68; 75,690
+// (2,713) 8.92, 8.93, 8.91; 109,744 (2,965) 12.01, 11.95, 11.93; 291,359 53.7, 52.2, 51.8.
 constexpr int kKB = 224;               // most of any front
-constexpr int kKBLargeFront = 1400;
+constexpr int kKBLargeFront = 2048;
 #if defined(__CUDACC__)
 __host__ __device__
 #endif
