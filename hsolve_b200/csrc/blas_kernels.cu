@@ -26,13 +26,13 @@ namespace {
 // lanes: the entries of a row are read by neighbouring lanes, the gathers of neighbouring rows fall into the same
 // lines, and the partial sums take two shuffle steps. A curl-curl row has at most 13 entries: a warp per row left
 // 19 lanes idle and spent most of its time in five-step reductions (the call for the residual of 8 columns at
-// n = 21,660: 135 us, now 24).
+// n = 21,660: 135 us, now 23).
 //
 // Longer rows want more lanes: chunks above most_entries a row take sixteen lanes a row, rows above kLongRow a
 // warp each. With four lanes up to 128 entries and the warp's own eight rows one after another above, the
-// residual of 8 columns took 33 us at n = 3,000 with 64 entries a row (now 25; a warp per row 41), 112 with 192
-// entries (39; 56) and 1,104 where 8 of the 3,000 rows were full (162; 215); a product of 8 columns 524 us there
-// (67; 95).
+// residual of 8 columns took 33 us at n = 3,000 with 64 entries a row (now 24; a warp per row 42), 107 with 192
+// entries (38; 57) and 1,104 where 8 of the 3,000 rows were full (160; 214); a product of 8 columns 523 us there
+// (60; 95).
 constexpr int kRowThreads = 256;
 constexpr int kRowWarps = kRowThreads / 32;
 constexpr int kChunk = kRowThreads / 4, kSmallChunk = kRowThreads / 16;
@@ -41,8 +41,8 @@ constexpr int kLongRow = 512;
 
 // Entries a row up to which a chunk takes four lanes a row. In few rows they leave the device idle (n = 3,000,
 // residual of 8 columns, four and sixteen lanes: 13 entries 22 and 20 us, 30 entries 28 and 21; one column
-// 17.4 and 18.4, 17.3 and 17.7); in many rows they move less (n = 100,000, 8 columns, 96 entries: 188 and
-// 308 us, 128 entries 231 and 397; a product of one column 43 and 39, 52 and 44).
+// 17.4 and 18.4, 17.3 and 17.7); in many rows they move less (n = 100,000, 8 columns, 96 entries: 173 and
+// 308 us, 128 entries 211 and 397; a product of one column 42 and 39, 51 and 44).
 template <int P>
 __device__ __forceinline__ int most_entries(int chunk) {
   return chunk == kSmallChunk ? 24 : (P == 1 ? 96 : 128);
@@ -120,44 +120,30 @@ struct GroupCols {
 // by four lanes (i may lie beyond), or wide(row0, end) for a chunk of many entries; entries(a, b) are those of the
 // rows [a, b). Both leave out the long rows, which take a warp each, long_row(i): a CTA's warps share those of
 // eight groups spread over the matrix, so that neighbouring long rows meet as many CTAs as there are groups of
-// them (1,000 rows of 1,000 entries at the end of 100,000 of 13, a product of 8 columns: 364 us by the warps of
-// the rows' own chunks, now 85).
+// them (1,000 rows of 1,000 entries at the end of 100,000 of 13, a product of 8 columns: 365 us by the warps of
+// the rows' own chunks, now 83).
 template <int P, class Span, class Entries, class Quad, class Wide, class LongRow>
 __device__ __forceinline__ void for_rows(std::int64_t n, int chunk, Span&& span, Entries&& entries, Quad&& quad,
                                          Wide&& wide, LongRow&& long_row) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int group_rows = chunk / kRowWarps, group_lanes = kRowThreads / chunk;
-  const std::int64_t step = gridDim.x * static_cast<std::int64_t>(chunk);
-  const auto group = [&](std::int64_t base, int w) {
-    return base + (w * static_cast<std::int64_t>(gridDim.x) + blockIdx.x) * group_rows;
-  };
-  bool some = false;
-  for (std::int64_t base = 0; base < n; base += step) {
-    const std::int64_t row0 = base + blockIdx.x * static_cast<std::int64_t>(chunk);
-    const std::int64_t end = row0 + chunk < n ? row0 + chunk : n, i = row0 + (threadIdx.x >> 2);
-    const std::int64_t k = group(base, warp) + lane / group_lanes;
-    // (all row pointers are read at once, before the chunk's kind is known)
-    const std::int64_t there = k < n ? entries(k, k + 1) : 0;
-    const auto mine = span(i, end);
-    if (row0 < n) {
-      if (entries(row0, end) > most_entries<P>(chunk) * (end - row0)) wide(row0, end);
-      else if (__any_sync(0xffffffffu, i < end)) quad(i, mine);
-    }
-    some |= there > kLongRow;
-  }
-  if (!__syncthreads_or(some)) return;
+  const auto group = [&](int w) { return (w * static_cast<std::int64_t>(gridDim.x) + blockIdx.x) * group_rows; };
+  const std::int64_t row0 = blockIdx.x * static_cast<std::int64_t>(chunk), end = row0 + chunk < n ? row0 + chunk : n;
+  const std::int64_t i = row0 + (threadIdx.x >> 2), k = group(warp) + lane / group_lanes;
+  // (all row pointers are read at once, before the chunk's kind is known)
+  const auto mine = span(i, end);
+  const bool is_long = k < n && entries(k, k + 1) > kLongRow;
+  if (entries(row0, end) > most_entries<P>(chunk) * (end - row0)) wide(row0, end);
+  else if (__any_sync(0xffffffffu, i < end)) quad(i, mine);
+  if (!__syncthreads_or(is_long)) return;
   __shared__ unsigned mask[kRowWarps];
-  for (std::int64_t base = 0; base < n; base += step) {
-    const std::int64_t k = group(base, warp) + lane / group_lanes;
-    const unsigned mine = __ballot_sync(0xffffffffu, lane % group_lanes == 0 && k < n && entries(k, k + 1) > kLongRow);
-    if (lane == 0) mask[warp] = mine;
-    __syncthreads();
-    int turn = 0;
-    for (int w = 0; w < kRowWarps; ++w)
-      for (unsigned m = mask[w]; m; m &= m - 1)
-        if (turn++ % kRowWarps == warp) long_row(group(base, w) + (__ffs(m) - 1) / group_lanes);
-    __syncthreads();  // the masks are written again
-  }
+  const unsigned found = __ballot_sync(0xffffffffu, lane % group_lanes == 0 && is_long);
+  if (lane == 0) mask[warp] = found;
+  __syncthreads();
+  int turn = 0;
+  for (int w = 0; w < kRowWarps; ++w)
+    for (unsigned m = mask[w]; m; m &= m - 1)
+      if (turn++ % kRowWarps == warp) long_row(group(w) + (__ffs(m) - 1) / group_lanes);
 }
 
 struct SpmmArgs {
@@ -514,26 +500,27 @@ __global__ void __launch_bounds__(kRowThreads, P == 1 ? 4 : 3)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane < P) part[warp][lane] = 0.0;
   __syncwarp();
-  double om[GroupCols<P, 4>::kCols] = {};
   const auto entries = [&](std::int64_t a, std::int64_t b) {
     const std::int64_t in_a = g.arp[b] - g.arp[a], in_b = g.brp ? g.brp[b] - g.brp[a] : 0;
     return in_a > in_b ? in_a : in_b;
   };
   for_rows<P>(g.n, chunk, [&](std::int64_t i, std::int64_t end) { return ResidualSpan(g, i, end); }, entries,
            [&](std::int64_t i, const ResidualSpan& e) {
-             residual_row<P, 4, 4>(g, i, e.a0, e.a1, e.b0, e.b1, e.mine,
-                                   [&](int u, double w) { om[u] = fmax(om[u], w); });
+             double om[GroupCols<P, 4>::kCols] = {};
+             residual_row<P, 4, 4>(g, i, e.a0, e.a1, e.b0, e.b1, e.mine, [&](int u, double w) { om[u] = w; });
+             keep_maxima<P, 4>(om, part[warp]);
            },
            [&](std::int64_t row0, std::int64_t end) { residual_wide_rows<P>(g, row0, end, part[warp]); },
            [&](std::int64_t i) { residual_long_row<P>(g, i, part[warp]); });
-  keep_maxima<P, 4>(om, part[warp]);
   if (omega) {
     // one atomic per column and CTA
     __syncthreads();
     if (threadIdx.x < P && static_cast<int>(threadIdx.x) < g.p) {
       double w = 0.0;
       for (int q = 0; q < kRowWarps; ++q) w = fmax(w, part[q][threadIdx.x]);
-      if (w > 0.0) atomic_max_nonneg(&omega[threadIdx.x], w);
+      // (it only grows: most CTAs find a larger one there)
+      const double there = __longlong_as_double(static_cast<long long>(__ldcg(&omega[threadIdx.x])));
+      if (w > there) atomic_max_nonneg(&omega[threadIdx.x], w);
     }
   }
 }
@@ -604,16 +591,15 @@ int grid_for(std::int64_t work, int threads) {
   return static_cast<int>(b < 1 ? 1 : (b > 148 * 32 ? 148 * 32 : b));
 }
 
-// rows of a CTA's chunk, and the CTAs: chunks are short while the matrix has too few rows for three CTAs an SM
+// rows of a CTA's chunk: short while the matrix has too few rows for three CTAs an SM
 int row_chunk(std::int64_t n) { return n <= kSmallRows ? kSmallChunk : kChunk; }
-int row_grid(std::int64_t n) { return grid_for(n * (kRowThreads / row_chunk(n)), kRowThreads); }
 
 }  // namespace
 
 void spmm(const CsrDev& M, const double* x, std::int64_t ldx, double* y, std::int64_t ldy, int p, double alpha,
           double beta, cudaStream_t s) {
   if (p <= 0 || M.n == 0) return;
-  const int blocks = row_grid(M.n), chunk = row_chunk(M.n);
+  const int chunk = row_chunk(M.n), blocks = static_cast<int>((M.n + chunk - 1) / chunk);
   for (int c0 = 0; c0 < p; c0 += 8) {
     const int pc = p - c0 < 8 ? p - c0 : 8;
     const double* xc = x + c0 * ldx;
@@ -741,7 +727,7 @@ void shifted_residual(const CsrDev& A, const CsrDev* B, double sigma, const doub
                       const double* y, std::int64_t ldy, double* r, std::int64_t ldr, int p, double* omega,
                       cudaStream_t s) {
   if (p <= 0 || A.n == 0) return;
-  const int blocks = row_grid(A.n), chunk = row_chunk(A.n);
+  const int chunk = row_chunk(A.n), blocks = static_cast<int>((A.n + chunk - 1) / chunk);
   if (omega) cuda_check(cudaMemsetAsync(omega, 0, static_cast<std::size_t>(p) * sizeof(double), s), "memset omega");
   for (int c0 = 0; c0 < p; c0 += 8) {
     const int pc = p - c0 < 8 ? p - c0 : 8;

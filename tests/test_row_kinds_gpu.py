@@ -79,8 +79,8 @@ def test_rows_of_all_kinds(n, p):
     _check(_matrix(counts, n, rng), _matrix(other, n, rng), p, rng)
 
 
-def test_many_rows_a_cta():
-    """More rows than one pass of the largest grid takes: 4,736 chunks of 64."""
+def test_many_chunks():
+    """Long rows at both ends of 4,738 chunks of 64."""
     n = 4736 * 64 + 77
     rng = np.random.default_rng(1)
     counts = np.full(n, 3)
