@@ -49,12 +49,14 @@ __device__ __forceinline__ int most_entries(int chunk) {
 }
 
 // f(value, column) for this lane's entries of the row [q0, q1): every G-th, kAhead of them read before the
-// gathers (a curl-curl row is one round of latencies).
+// gathers (a curl-curl row is one batch).
 template <int G, int kAhead, bool kWhole, class Fn>
 __device__ __forceinline__ void group_entries(std::int64_t q0, std::int64_t q1, const std::int32_t* ci, const double* v,
                                               Fn&& f) {
   std::int64_t q = q0 + (threadIdx.x & (G - 1));
-  if constexpr (G > 4 && kWhole) {  // (rows of many rounds: the whole ones without tests)
+  // rows of many batches: the whole ones without tests (not with eight columns, whose sums leave no registers for
+  // a second copy of the batch: a product of 3,000 rows with 128 entries took 24 us, 18 without)
+  if constexpr (G > 4 && kWhole) {
     for (; q + G * (kAhead - 1) < q1; q += G * kAhead) {
       double a[kAhead];
       std::int32_t j[kAhead];

@@ -14,7 +14,7 @@ SMALL = 444 * 16  # most rows that are taken in chunks of 16
 
 
 def _matrix(counts, n, rng):
-    """Row i has counts[i] entries, in consecutive columns (around the diagonal's place) in a shuffled order."""
+    """Row i has counts[i] entries, in consecutive columns around the diagonal (cyclically)."""
     counts = np.minimum(counts, n)
     rows = np.repeat(np.arange(n), counts)
     start = np.arange(n) - counts // 2
